@@ -30,6 +30,7 @@
 // all CTAs stop together once every pair is at or below the threshold -- no
 // host round trip.  A barrier wait that exceeds its poll budget records
 // TM_DEV_ERR_TIMEOUT in the device status word and makes every CTA leave.
+#include <algorithm>
 #include <cmath>
 
 #include "tm_tma.cuh"
@@ -329,6 +330,376 @@ __global__ void __launch_bounds__(kSkThreads, 2) sk_solve_kernel(SkArgs A) {
     if (blockIdx.x == 0 && threadIdx.x == 0) A.ctl->iterations = it;
 }
 
+// ----------------------------------------------------- resident row slabs
+// The tile kernel above gives a CTA 128 matrix rows, so a problem of a few
+// hundred points keeps a handful of SMs busy and every half-step waits for
+// their 128-row contractions.  Where the matrix is small, sk_slab_kernel cuts
+// it into slabs of 8 to 32 rows instead: CTA (c, g) keeps rows [c R, c R + R) of K
+// and of K^T in its shared memory for the whole solve and updates the pairs of
+// group g, one CTA per SM, so a half-step reads only the other side's scalings
+// (from L2) and costs one barrier among the CTAs of the group (pairs never
+// meet; with a stopping test the decision is common and so is the barrier).
+//
+// Bound: the barrier and the L2 round trips of the scalings, not arithmetic
+// (16 pairs x 784 points: 0.2 us of FMAs per CTA and half-step, 5.4 us taken).
+// Measured per iteration, tile kernel -> slabs (GB300, whole solves of 50): scaling
+// form 16 x 784 88 -> 10.9 us, 16 x 1600 172 -> 26 us, 48 x 64 20 -> 8 us, 256 x 784
+// 136 -> 71 us; log form 16 x 784 127 -> 18 us, 31 x 1600 870 -> 115 us.
+//
+// W = ceil(d / 128) warps (at most 8) form a set that takes one tile of 8 rows x PT
+// pairs at a time, the 8 / W sets of a CTA different tiles.  A thread owns 4
+// columns (8 above 1024 points, V = 2: W = ceil(d / 256)) for all 8 rows and PT
+// pairs: the scalings go from L2 straight into its registers.  The 8 x PT partial sums of
+// the set's threads are reduced by transposing butterflies (62 shuffles for 64
+// sums) and across the warps in shared memory; then one thread per (row, pair)
+// finishes the output.  The log form takes the maximum of every (row, pair) in a
+// first pass and sums 2^(z - max) in a second.
+constexpr int kSlabRows = 8;       // rows per tile
+constexpr int kSlabMaxCtas = 160;  // CTAs of a launch (residual partials are sized for these)
+constexpr int kSlabWarps = kSkThreads / 32;
+constexpr int kSlabMaxGroups = 60;  // arrival counters in the control block
+
+template <bool LOG, int V>
+struct SlabTile {
+    static constexpr int PT = LOG || V > 1 ? 4 : 8;  // pairs per tile
+    static constexpr int N = kSlabRows * PT;         // sums per thread
+    static constexpr int kCols = 128 * V;            // columns per warp
+};
+
+struct SlabShape {
+    int rows;    // R: rows per CTA, a multiple of kSlabRows
+    int ctas;    // CTAs of a group
+    int groups;  // pair groups
+    int pairs;   // pairs per group
+    int pitch;   // floats per slab row (d rounded up to 4)
+    size_t smem;
+};
+
+// Arrival counter barrier: the count only grows, so a CTA arrives with one add and
+// waits for `target` (modulo 2^32).  Bounded like grid_barrier_bounded.
+__device__ inline bool slab_barrier(SkControl *ctl, int *counter, unsigned target, int *status,
+                                    long long spin_limit) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(counter, 1);
+        int ok = 1;
+        long long polls = 0;
+        volatile int *abort = &ctl->abort;
+        for (;;) {
+            unsigned cnt;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cnt) : "l"(counter) : "memory");
+            if ((int)(cnt - target) >= 0) break;
+            if (++polls > spin_limit || ((polls & 63) == 0 && *abort)) {
+                ok = 0;
+                break;
+            }
+        }
+        if (!ok) {
+            atomicExch(&ctl->abort, 1);
+            if (status) atomicExch(status, TM_DEV_ERR_TIMEOUT);
+        }
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// Barrier of the `threads` threads of warp set `set` (hardware barriers 1 .. 8).
+__device__ __forceinline__ void set_sync(int set, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(set + 1), "r"(threads) : "memory");
+}
+
+// v[0..N) of every lane -> sums (or maxima) over the 32 lanes: lane l is left with
+// entries l (N / 32) + k, k < N / 32, in v[k].
+template <int N, bool MAX>
+__device__ __forceinline__ void transpose_reduce(float (&v)[N]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16, half = N / 2; o > 0; o >>= 1, half >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < half; k++) {
+            const float send = up ? v[k] : v[k + half], keep = up ? v[k + half] : v[k];
+            const float got = __shfl_xor_sync(0xffffffffu, send, o);
+            v[k] = MAX ? fmaxf(keep, got) : keep + got;
+        }
+    }
+}
+
+// One half-step of the CTA's rows: out[b, i] for i in [i0, i0 + R), b in [b_lo, b_hi).
+template <bool LOG, int V>
+__device__ __forceinline__ void slab_half(const SkArgs &A, const SlabShape &sh, int i0, int b_lo, int b_hi,
+                                          const float *slab, float *red_all, const float *__restrict__ num,
+                                          const float *scale, float *out, double *partial_row) {
+    constexpr int PT = SlabTile<LOG, V>::PT, N = SlabTile<LOG, V>::N, COLS = SlabTile<LOG, V>::kCols;
+    const int d = A.d, pitch = sh.pitch;
+    const int W = (d + COLS - 1) / COLS, sets = kSlabWarps / W, set = (threadIdx.x >> 5) / W;
+    if (set >= sets) return;  // left-over warps (they meet the others at the next block barrier)
+    const int st = threadIdx.x - set * W * 32, warp = st >> 5, lane = st & 31, nthr = W * 32;
+    float *red = red_all + (size_t)set * (W + 1) * N;  // [W][N] partial sums, then N maxima
+    const float sfill = LOG ? -INFINITY : 0.0f;
+    // this thread's columns: 4 (st + v W 32) .. + 3, v < V
+    auto load_scale = [&](float4(&x)[PT][V], int b0) {
+#pragma unroll
+        for (int p = 0; p < PT; p++)
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                const int j = 4 * (st + v * nthr);
+                float4 q = make_float4(sfill, sfill, sfill, sfill);
+                if (b0 + p < b_hi && j < d) {
+                    // u and v are rewritten by other CTAs during the launch: L2 loads, never L1
+                    const float *src = scale + (size_t)(b0 + p) * d + j;
+                    if (A.vec) {
+                        q = __ldcg(reinterpret_cast<const float4 *>(src));
+                    } else {
+                        q.x = __ldcg(src);
+                        if (j + 1 < d) q.y = __ldcg(src + 1);
+                        if (j + 2 < d) q.z = __ldcg(src + 2);
+                        if (j + 3 < d) q.w = __ldcg(src + 3);
+                    }
+                }
+                x[p][v] = q;
+            }
+    };
+    const int ntiles = (b_hi - b_lo + PT - 1) / PT;
+    float4 sv[PT][V], nx[PT][V];
+    if (!LOG && set < ntiles) load_scale(nx, b_lo + set * PT);
+    for (int t = set; t < ntiles; t += sets) {
+        const int b0 = b_lo + t * PT;
+        if (LOG) load_scale(nx, b0);
+#pragma unroll
+        for (int p = 0; p < PT; p++)
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                sv[p][v] = nx[p][v];
+                if (LOG) {
+                    sv[p][v].x *= kLog2e;
+                    sv[p][v].y *= kLog2e;
+                    sv[p][v].z *= kLog2e;
+                    sv[p][v].w *= kLog2e;
+                }
+            }
+        if (!LOG && t + sets < ntiles) load_scale(nx, b0 + sets * PT);  // in flight behind this tile
+        for (int r0 = 0; r0 < sh.rows && i0 + r0 < d; r0 += kSlabRows) {
+            // the outputs this thread finishes: entry e = 8 p + r of the tile
+            constexpr int kOwn = N / 32;  // at least 32 threads
+            float nu[kOwn], old[kOwn];
+#pragma unroll
+            for (int k = 0; k < kOwn; k++) {
+                const int e = st + k * nthr, i = i0 + r0 + (e & 7), b = b0 + (e >> 3);
+                const bool own = e < N && i < d && b < b_hi;
+                nu[k] = own ? num[(size_t)b * d + i] : 0.0f;
+                old[k] = own && partial_row ? __ldcg(out + (size_t)b * d + i) : 0.0f;
+            }
+            const float *rows = slab + (size_t)r0 * pitch;
+            float acc[N];
+            if (LOG) {
+#pragma unroll
+                for (int k = 0; k < N; k++) acc[k] = kNoMax;
+#pragma unroll
+                for (int v = 0; v < V; v++) {
+                    // (at most one turn: the loop keeps the row loads of one v from being moved
+                    // across the others', which would not fit in registers)
+                    for (int j = 4 * (st + v * nthr); j < pitch; j += 4 * V * nthr)
+#pragma unroll
+                    for (int r = 0; r < kSlabRows; r++) {
+                        const float4 kv = *reinterpret_cast<const float4 *>(rows + (size_t)r * pitch + j);
+#pragma unroll
+                        for (int p = 0; p < PT; p++)
+                            acc[p * kSlabRows + r] =
+                                fmaxf(acc[p * kSlabRows + r], fmaxf(fmaxf(kv.x + sv[p][v].x, kv.y + sv[p][v].y),
+                                                                    fmaxf(kv.z + sv[p][v].z, kv.w + sv[p][v].w)));
+                    }
+                }
+                transpose_reduce<N, true>(acc);
+#pragma unroll
+                for (int k = 0; k < N / 32; k++) red[warp * N + lane * (N / 32) + k] = acc[k];
+                set_sync(set, nthr);
+                if (st < N) {
+                    float m = kNoMax;
+                    for (int w = 0; w < W; w++) m = fmaxf(m, red[w * N + st]);
+                    red[W * N + st] = m;
+                }
+                set_sync(set, nthr);
+            }
+#pragma unroll
+            for (int k = 0; k < N; k++) acc[k] = 0.0f;
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                for (int j = 4 * (st + v * nthr); j < pitch; j += 4 * V * nthr)
+#pragma unroll
+                for (int r = 0; r < kSlabRows; r++) {
+                    const float4 kv = *reinterpret_cast<const float4 *>(rows + (size_t)r * pitch + j);
+#pragma unroll
+                    for (int p = 0; p < PT; p++) {
+                        float x = acc[p * kSlabRows + r];
+                        if (!LOG) {
+                            x = fmaf(kv.x, sv[p][v].x, x);
+                            x = fmaf(kv.y, sv[p][v].y, x);
+                            x = fmaf(kv.z, sv[p][v].z, x);
+                            x = fmaf(kv.w, sv[p][v].w, x);
+                        } else {
+                            const float M = red[W * N + p * kSlabRows + r];
+                            x += (ex2((kv.x + sv[p][v].x) - M) + ex2((kv.y + sv[p][v].y) - M)) +
+                                 (ex2((kv.z + sv[p][v].z) - M) + ex2((kv.w + sv[p][v].w) - M));
+                        }
+                        acc[p * kSlabRows + r] = x;
+                    }
+                }
+            }
+            transpose_reduce<N, false>(acc);
+#pragma unroll
+            for (int k = 0; k < N / 32; k++) red[warp * N + lane * (N / 32) + k] = acc[k];
+            set_sync(set, nthr);
+#pragma unroll
+            for (int k = 0; k < kOwn; k++) {
+                const int e = st + k * nthr, i = i0 + r0 + (e & 7), b = b0 + (e >> 3);
+                if (e >= N) break;  // N is a multiple of 32: whole warps leave
+                float sum = 0.0f, res = 0.0f;
+                for (int w = 0; w < W; w++) sum += red[w * N + e];
+                const bool own = i < d && b < b_hi;
+                if (own) {
+                    float o;
+                    if (!LOG) {
+                        if (partial_row) res = fabsf(nu[k] - old[k] * sum);
+                        o = nu[k] / (sum + 1e-12f);
+                    } else {
+                        const float M = red[W * N + e];
+                        const bool none = !(M > kNoMax);  // every term was -inf
+                        const float lse2 = M + log2f(sum);
+                        if (partial_row) {
+                            const float plan_row = none ? 0.0f : ex2(fmaf(old[k], kLog2e, lse2));
+                            res = fabsf(ex2(nu[k] * kLog2e) - plan_row);
+                        }
+                        o = none ? -INFINITY : nu[k] - lse2 * kLn2;
+                    }
+                    out[(size_t)b * d + i] = o;
+                }
+                if (partial_row) {  // 8 adjacent lanes hold the tile's rows of one pair
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) res += __shfl_xor_sync(0xffffffffu, res, o);
+                    if ((e & 7) == 0 && own) {
+                        if (r0 == 0) partial_row[b] = (double)res;
+                        else partial_row[b] += (double)res;  // this thread's own earlier store
+                    }
+                }
+            }
+            set_sync(set, nthr);  // the partial sums are rewritten by the next tile
+        }
+    }
+}
+
+template <bool LOG, int V>
+__global__ void __launch_bounds__(kSkThreads, 1) sk_slab_kernel(SkArgs A, SlabShape sh) {
+    extern __shared__ __align__(16) float slab_smem[];
+    const int rows = sh.rows, pitch = sh.pitch;
+    float *su = slab_smem;                              // rows of K (u-update)
+    float *sv = slab_smem + (size_t)rows * pitch;       // rows of K^T (v-update)
+    float *red = slab_smem + (size_t)2 * rows * pitch;  // partial sums and maxima
+    const int slab = blockIdx.x % sh.ctas, group = blockIdx.x / sh.ctas;
+    const int i0 = slab * rows, d = A.d;
+    const int b_lo = group * sh.pairs, b_hi = min(A.n, b_lo + sh.pairs);
+    const float fill = LOG ? -INFINITY : 0.0f;
+    for (int r = 0; r < rows; r++) {
+        const int i = i0 + r;
+        for (int j = threadIdx.x; j < pitch; j += kSkThreads) {
+            float x = fill, y = fill;
+            if (i < d && j < d) {
+                if (A.mat) {
+                    x = A.mat[(size_t)i * d + j];
+                    y = A.mat_t[(size_t)i * d + j];
+                } else {  // the line cost is symmetric
+                    x = LOG ? line_cost(i, j) : expf(-line_cost(i, j) * A.inv_eps);
+                    y = x;
+                }
+                if (LOG) {
+                    x *= A.mscale;
+                    y *= A.mscale;
+                }
+            }
+            su[r * pitch + j] = x;
+            sv[r * pitch + j] = y;
+        }
+    }
+    __syncthreads();
+    // with a stopping test every CTA takes part in one decision; without, a group is on its own
+    const bool common = A.check_every > 0;
+    int *counter = &A.ctl->pad[common ? 0 : group];
+    const unsigned arrivals = common ? gridDim.x : (unsigned)sh.ctas;
+    unsigned target = 0;
+    int check = 0, it = 0;
+    for (; it < A.max_iter; it++) {
+        const bool checking = common && (it + 1) % A.check_every == 0;
+        slab_half<LOG, V>(A, sh, i0, b_lo, b_hi, su, red, A.num_u, A.v, A.u,
+                       checking ? A.partial + (size_t)slab * A.n : nullptr);
+        if (!slab_barrier(A.ctl, counter, target += arrivals, A.status, A.spin_limit)) return;
+        if (checking) {  // per-pair residual sums, one warp per pair, fixed order
+            const int warps = gridDim.x * kSlabWarps;
+            const int lane = threadIdx.x & 31;
+            for (int b = blockIdx.x * kSlabWarps + (threadIdx.x >> 5); b < A.n; b += warps) {
+                double s = 0.0;
+                for (int r = lane; r < sh.ctas; r += 32) s += __ldcg(A.partial + (size_t)r * A.n + b);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) {
+                    A.err[b] = s;
+                    if (!(s <= (double)A.threshold)) atomicOr(&A.notconv[check], 1);
+                }
+            }
+        }
+        slab_half<LOG, V>(A, sh, i0, b_lo, b_hi, sv, red, A.num_v, A.u, A.v, nullptr);
+        if (!slab_barrier(A.ctl, counter, target += arrivals, A.status, A.spin_limit)) return;
+        if (checking) {
+            const bool stop = *((volatile int *)&A.notconv[check]) == 0;
+            check++;
+            if (stop) {
+                it++;
+                break;
+            }
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.ctl->iterations = it;
+}
+
+// The shape the slab kernel runs an (n, d) problem in, or false where the tile kernel
+// keeps it.  Of R = 8 .. 32 rows per CTA that fit in shared memory the one with the
+// fewest tile rounds per half-step wins, on a tie the larger (fewer CTAs meet at a
+// barrier, each scaling is read by fewer of them).  A round costs about 1.4 us (log
+// form 2 us, 2.8 us above 1024 points), the tile kernel 0.085 (0.28) us per column and
+// wave: many pairs over many points stay with it (scaling 256 x 1700: 282 us an
+// iteration against 352 in slabs; log 512 x 1200: 714 against 895).
+template <bool LOG, int V>
+inline bool slab_shape(int64_t n, int64_t d, int sms, SlabShape *out) {
+    constexpr int PT = SlabTile<LOG, V>::PT, N = SlabTile<LOG, V>::N;
+    const int64_t W = ceil_div(d, (int64_t)SlabTile<LOG, V>::kCols), sets = kSlabWarps / W;
+    if (W > kSlabWarps) return false;
+    int64_t best = 0;
+    for (int rows = kSlabRows; rows <= 4 * kSlabRows; rows += kSlabRows) {
+        SlabShape s;
+        s.rows = rows;
+        s.ctas = (int)ceil_div(d, (int64_t)rows);
+        s.pitch = (int)((d + 3) & ~(int64_t)3);
+        s.smem = ((size_t)2 * rows * s.pitch + (size_t)sets * (W + 1) * N) * sizeof(float);
+        if (s.ctas > sms || s.smem > (size_t)224 * 1024) continue;
+        const int64_t tiles = ceil_div(n, PT);
+        int64_t groups = std::min<int64_t>(std::min<int64_t>(sms / s.ctas, tiles), kSlabMaxGroups);
+        const int64_t tiles_per = ceil_div(tiles, groups);
+        s.groups = (int)ceil_div(tiles, tiles_per);
+        s.pairs = (int)(tiles_per * PT);
+        const int64_t rounds = (rows / kSlabRows) * ceil_div(tiles_per, sets);
+        if (best == 0 || rounds <= best) {
+            best = rounds;
+            *out = s;
+        }
+    }
+    // a round against d columns of the tile kernel's waves
+    const int64_t waves = ceil_div(ceil_div(d, kSkRows) * ceil_div(n, 64), 2 * (int64_t)sms);
+    return best > 0 && best * (LOG ? (V > 1 ? 10 : 7) : 16) < d * waves;
+}
+
 // K = exp(-C / eps) and K^T (scaling form), or C^T alone (log form, EXP = false),
 // through 32 x 32 shared-memory tiles so both writes are coalesced.  inv_eps is
 // the float32 reciprocal of eps: torch evaluates a CUDA tensor divided by a
@@ -447,15 +818,109 @@ __global__ void __launch_bounds__(kSkThreads)
     }
 }
 
+// The same sums for problems whose 128-row x 16-pair blocks would leave SMs idle: a
+// CTA takes 4 rows x 4 pairs with 16 lanes across the columns of each, reading the
+// cost rows and log v through L1 (float4 where aligned).  fp32 sums over 16 terms
+// are added in fp64, the lanes by shuffles.
+// 16 pairs x 784 points: 179 us with 7 blocks of the kernel above, 15 us with these.
+constexpr int kCostRows = 4, kCostPairs = 4, kCostLanes = 16;
+
+__global__ void __launch_bounds__(kSkThreads)
+    sk_cost_rows_kernel(const float *__restrict__ lu, const float *__restrict__ lv, const float *__restrict__ C,
+                        const float *__restrict__ a, int n, int d, float inv_eps, bool vec,
+                        double *__restrict__ cost_part, double *__restrict__ err_part) {
+    __shared__ double s_cost[kCostRows][kCostPairs], s_err[kCostRows][kCostPairs];
+    const int lane = threadIdx.x & (kCostLanes - 1), cell = threadIdx.x / kCostLanes;
+    const int row = cell % kCostRows, pair = cell / kCostRows;
+    const int pair_blocks = (n + kCostPairs - 1) / kCostPairs;
+    const int rb = blockIdx.x / pair_blocks, pb = blockIdx.x % pair_blocks;
+    const int i = rb * kCostRows + row, b = pb * kCostPairs + pair;
+    double cacc = 0.0, racc = 0.0;
+    if (i < d && b < n) {
+        const float x = lu[(size_t)b * d + i];
+        const float *crow = C ? C + (size_t)i * d : nullptr;
+        const float *vrow = lv + (size_t)b * d;
+        for (int j0 = 4 * lane; j0 < d; j0 += 16 * kCostLanes) {
+            float cs = 0.0f, rs = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int j = j0 + 4 * kCostLanes * q;
+                if (j >= d) break;
+                float c[4], v[4];
+                if (vec) {
+                    const float4 v4 = *reinterpret_cast<const float4 *>(vrow + j);
+                    v[0] = v4.x, v[1] = v4.y, v[2] = v4.z, v[3] = v4.w;
+                    if (crow) {
+                        const float4 c4 = *reinterpret_cast<const float4 *>(crow + j);
+                        c[0] = c4.x, c[1] = c4.y, c[2] = c4.z, c[3] = c4.w;
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; e++) c[e] = line_cost(i, j + e);
+                    }
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const bool in = j + e < d;
+                        c[e] = !in ? 0.0f : (crow ? crow[j + e] : line_cost(i, j + e));
+                        v[e] = in ? vrow[j + e] : -INFINITY;
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float p = expf((x - c[e] * inv_eps) + v[e]);
+                    cs = fmaf(p, c[e], cs);
+                    rs += p;
+                }
+            }
+            cacc += (double)cs;
+            racc += (double)rs;
+        }
+    }
+#pragma unroll
+    for (int o = kCostLanes / 2; o > 0; o >>= 1) {
+        cacc += __shfl_xor_sync(0xffffffffu, cacc, o);
+        racc += __shfl_xor_sync(0xffffffffu, racc, o);
+    }
+    if (lane == 0) {
+        s_cost[row][pair] = cacc;
+        s_err[row][pair] = i < d && b < n ? fabs((double)a[(size_t)b * d + i] - racc) : 0.0;
+    }
+    __syncthreads();
+    if (threadIdx.x < kCostPairs && pb * kCostPairs + (int)threadIdx.x < n) {
+        double cs = 0.0, es = 0.0;
+#pragma unroll
+        for (int r = 0; r < kCostRows; r++) {
+            cs += s_cost[r][threadIdx.x];
+            es += s_err[r][threadIdx.x];
+        }
+        const size_t o = (size_t)rb * n + pb * kCostPairs + threadIdx.x;
+        cost_part[o] = cs;
+        err_part[o] = es;
+    }
+}
+
+// Which cost kernel takes an (n, d) problem: 128-row blocks once there is one for every
+// SM (4096 pairs x 64 points: 0.1 ms less than 4-row blocks), 4-row blocks below.
+inline bool cost_by_rows(int64_t n, int64_t d, int sms) {
+    return ceil_div(d, kSkRows) * ceil_div(n, 16) < (int64_t)sms;
+}
+
+// One warp per pair adds the row blocks in a fixed order.
 __global__ void sk_cost_reduce_kernel(const double *__restrict__ cost_part, const double *__restrict__ err_part,
                                       int n, int row_blocks, double *__restrict__ cost, double *__restrict__ err) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (b >= n) return;
     double c = 0.0, e = 0.0;
-    for (int r = 0; r < row_blocks; r++) {
+    for (int r = lane; r < row_blocks; r += 32) {
         c += cost_part[(size_t)r * n + b];
         e += err_part[(size_t)r * n + b];
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+    }
+    if (lane != 0) return;
     if (cost) cost[b] = c;
     if (err) err[b] = e;
 }
@@ -573,6 +1038,31 @@ int check_nd(int64_t n, int64_t d) {
 
 bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
+// Launches the slab kernel where the problem has its shape (the tuning table does not
+// reach these: its variants are shapes of the tile kernel).
+template <bool LOG, int V>
+bool sk_slab_launch(SkArgs &A, cudaStream_t s, int *st) {
+    SlabShape sh;
+    if (!slab_shape<LOG, V>(A.n, A.d, std::min(sm_count(), kSlabMaxCtas), &sh)) return false;
+    const void *kern = (const void *)sk_slab_kernel<LOG, V>;
+    auto run = [&]() -> int {
+        TM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+        TM_CHECK_CUDA(cudaMemsetAsync(A.ctl, 0, sizeof(SkControl), s));
+        void *params[] = {&A, &sh};
+        TM_CHECK_CUDA(cudaLaunchCooperativeKernel(kern, dim3(sh.ctas * sh.groups), dim3(kSkThreads), params, sh.smem, s));
+        TM_LAUNCH_CHECK("sk_slab_kernel");
+        return TM_OK;
+    };
+    *st = run();
+    return true;
+}
+
+bool sk_slab(bool log_form, SkArgs &A, cudaStream_t s, int *st) {
+    const bool wide = A.d > kSlabWarps * SlabTile<false, 1>::kCols;
+    if (log_form) return wide ? sk_slab_launch<true, 2>(A, s, st) : sk_slab_launch<true, 1>(A, s, st);
+    return wide ? sk_slab_launch<false, 2>(A, s, st) : sk_slab_launch<false, 1>(A, s, st);
+}
+
 // The persistent solver on caller-provided state.  control: 256-byte control
 // block; partial/err/notconv only when check_every > 0.
 int sk_launch(bool log_form, SkArgs A, cudaStream_t s) {
@@ -583,6 +1073,7 @@ int sk_launch(bool log_form, SkArgs A, cudaStream_t s) {
     A.spin_limit = grid_wait_budget();
     // autotuned variant: bit 0 = 64 pairs per tile (else 16), bit 1 = one CTA per SM
     // (else two); built-in: 64 pairs per tile above 24 pairs, two CTAs per SM
+    if (sk_slab(log_form, A, s, &st)) return st;
     const int variant = tune_variant(kTuneSinkhornF32, tune_class(kTuneSinkhornF32, A.n, A.d));
     const bool wide = variant < 0 ? A.n > 24 : (variant & 1) != 0;
     const void *kern;
@@ -611,7 +1102,7 @@ struct SkLayout {
 SkLayout sk_layout(int64_t n, int64_t d, bool log_form, int64_t max_iter, int64_t check_every, bool line) {
     SkLayout L{};
     const size_t dd = (size_t)d * d * sizeof(float), nd = (size_t)n * d * sizeof(float);
-    const size_t rblocks = (size_t)ceil_div(d, kSkRows);
+    const size_t rblocks = std::max((size_t)ceil_div(d, kSkRows), (size_t)kSlabMaxCtas);  // residual partials
     const size_t checks = check_every > 0 ? (size_t)(max_iter / check_every) + 1 : 1;
     size_t off = 0;
     L.mat = off;
@@ -630,10 +1121,14 @@ SkLayout sk_layout(int64_t n, int64_t d, bool log_form, int64_t max_iter, int64_
     off += align256(checks * sizeof(int));
     L.ctl = off;
     off += align256(sizeof(SkControl));
+    // (sized for the cost kernel with the more blocks where either may run: the SM count is a
+    // property of the device, not of the problem)
+    const size_t cblocks = cost_by_rows(n, d, kSlabMaxCtas) ? (size_t)ceil_div(d, kCostRows)
+                                                            : (size_t)ceil_div(d, kSkRows);
     L.cost_part = off;
-    off += align256(rblocks * n * sizeof(double));
+    off += align256(cblocks * n * sizeof(double));
     L.err_part = off;
-    off += align256(rblocks * n * sizeof(double));
+    off += align256(cblocks * n * sizeof(double));
     L.total = off;
     return L;
 }
@@ -649,13 +1144,21 @@ unsigned grid_for(size_t count) {
 
 int sk_cost(const float *lu, const float *lv, const float *C, const float *a, int64_t n, int64_t d, double epsilon,
             double *cost_part, double *err_part, double *cost, double *err, cudaStream_t s) {
-    const int64_t rblocks = ceil_div(d, kSkRows);
-    const unsigned blocks = (unsigned)(rblocks * ceil_div(n, 16));
-    sk_cost_kernel<<<blocks, kSkThreads, 0, s>>>(lu, lv, C, a, (int)n, (int)d, 1.0f / (float)epsilon, cost_part,
-                                                 err_part);
-    TM_LAUNCH_CHECK("sk_cost_kernel");
-    sk_cost_reduce_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(cost_part, err_part, (int)n, (int)rblocks, cost,
-                                                                     err);
+    int64_t rblocks;
+    const float inv_eps = 1.0f / (float)epsilon;
+    if (cost_by_rows(n, d, std::min(sm_count(), kSlabMaxCtas))) {
+        rblocks = ceil_div(d, kCostRows);
+        const bool vec = (d % 4) == 0 && aligned16(lv) && aligned16(C);
+        sk_cost_rows_kernel<<<(unsigned)(rblocks * ceil_div(n, kCostPairs)), kSkThreads, 0, s>>>(
+            lu, lv, C, a, (int)n, (int)d, inv_eps, vec, cost_part, err_part);
+        TM_LAUNCH_CHECK("sk_cost_rows_kernel");
+    } else {
+        rblocks = ceil_div(d, kSkRows);
+        sk_cost_kernel<<<(unsigned)(rblocks * ceil_div(n, 16)), kSkThreads, 0, s>>>(lu, lv, C, a, (int)n, (int)d,
+                                                                                    inv_eps, cost_part, err_part);
+        TM_LAUNCH_CHECK("sk_cost_kernel");
+    }
+    sk_cost_reduce_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, s>>>(cost_part, err_part, (int)n, (int)rblocks, cost, err);
     TM_LAUNCH_CHECK("sk_cost_reduce_kernel");
     return TM_OK;
 }
