@@ -493,18 +493,15 @@ int check_edt_args(const void *input, int in_dtype, const Geometry &g, const flo
 }  // namespace
 }  // namespace tmc
 
-static bool unit_sampling(int ndim, const float *sampling) {
-    if (!sampling) return true;
-    for (int d = 0; d < ndim; d++)
-        if (sampling[d] != 1.0f) return false;
-    return true;
-}
-
 extern "C" size_t tm_edt_workspace_size(int64_t batch, int ndim, const int64_t *shape, const float *sampling) {
     tmc::Geometry g;
     if (tmc::make_geometry(batch, ndim, shape, &g) != TM_OK) return 0;
-    if (tmc::edt_compact_eligible(g, unit_sampling(ndim, sampling))) return tmc::edt_compact_workspace(g);
-    return tmc::plan_edt(g).total;
+    tmc::EdtSpacing sp;
+    const size_t general = tmc::plan_edt(g).total;
+    if (!tmc::edt_compact_eligible(g, sampling, &sp)) return general;
+    const size_t compact = tmc::edt_compact_workspace(g);
+    // (sampled calls keep the general passes' size, whichever passes take the spacing)
+    return sp.scaled && general > compact ? general : compact;
 }
 
 extern "C" int tm_edt(const void *input, int in_dtype, int64_t batch, int ndim, const int64_t *shape,
@@ -521,11 +518,12 @@ extern "C" int tm_edt(const void *input, int in_dtype, int64_t batch, int ndim, 
     if (sqdist && !unit) return fail(TM_ERR_INVALID_ARGUMENT, "squared integer distances need unit sampling");
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     cudaStream_t s = (cudaStream_t)stream;
-    if (edt_compact_eligible(g, unit)) {
+    EdtSpacing spacing;
+    if (edt_compact_eligible(g, sampling, &spacing)) {
         const size_t need = edt_compact_workspace(g);
         if (!workspace || workspace_bytes < need)
             return fail(TM_ERR_WORKSPACE, "workspace of %zu bytes required, got %zu", need, workspace_bytes);
-        return edt_compact_run(input, in_dtype, g, dist, indices, sqdist, ws, s);
+        return edt_compact_run(input, in_dtype, g, spacing, dist, indices, sqdist, ws, s);
     }
     EdtPlan pl = plan_edt(g);
     if (pl.total > 0 && (!workspace || workspace_bytes < pl.total))

@@ -1,7 +1,8 @@
-// Exact EDT fast path for 2-D and 3-D items with unit spacing (GB300, sm_103a).
+// Exact EDT fast path for 2-D and 3-D items with unit spacing, or spacings that
+// are binary fractions (GB300, sm_103a).
 //
 // Same result as the generic separable passes in edt.cu (scipy's feature
-// tie rule), restructured around four facts of the workload:
+// tie rule), restructured around these facts of the workload:
 //
 //  * Compact features.  After pass 0 a voxel's nearest site so far is
 //    (f0, own y, own x) and after pass 1 it is (f0, f1, own x), so the
@@ -9,29 +10,20 @@
 //    per voxel; squared distances are recomputed on chip instead of being
 //    stored: 2 + 4 bytes of intermediates per voxel.
 //
-//  * Bounded windows.  d(q) = min_p (q-p)^2 + g(p) is at most the best
-//    value among p = q-K .. q+K, and every minimiser -- ties included --
-//    lies within |q-p| <= isqrt(d(q)).  So the (2K+1)-candidate window is
-//    exact whenever its best value is below (K+1)^2 and is widened to the
-//    exact radius otherwise (K = 4 in pass 1, 2 in pass 2).  Lines that
-//    would need a radius above kFar run the Felzenszwalb-Huttenlocher lower
-//    envelope instead, so sparse inputs keep O(L) work per line.
+//  * Bounded windows, no serial chain per line: the passes of edt_lines.cuh.
 //
-//  * Packed keys.  A candidate is the 32-bit key (value << 5) | k, k its
-//    position in the window, so one unsigned min selects the smallest value
-//    and, among equal values, the lowest position -- the separable tie
-//    rule -- in two integer operations per candidate.
+//  * Dense backgrounds (unit spacing, 3-D): a bitmap search of the offsets
+//    around every voxel finds most features without any pass (below); the
+//    passes then run for the items it gave up.
 //
-//  * Coalescing and occupancy.  Passes 0 and 1 run along non-contiguous axes:
-//    a block stages 128 adjacent lines in shared memory with vectorised row
-//    loads, adjacent threads own adjacent lines, and each line is split over
-//    4 threads.  Pass 2 runs along the contiguous axis, one warp per line,
-//    4 voxels per lane with 16-byte loads and stores.
+//  * Ragged batches of 3-D items run passes 1 + 2 fused per plane in one
+//    cooperative launch.
 #include <cmath>
 #include <algorithm>
 #include <array>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -42,19 +34,15 @@ namespace {
 
 constexpr uint32_t kBig = 1u << 26;  // "no site"; eligible shapes keep every real value below it
 constexpr int kKeyShift = 5;         // key = value << 5 | window position
-constexpr int kCols = 128;           // lines per block in passes 0 and 1
-constexpr int kSegs = 4;             // threads per line in passes 0 and 1
-constexpr int kC2Warps = 8;          // lines per block in pass 2
 constexpr int kFar = 24;             // widest exact window before a line uses the envelope
 constexpr int kNear1 = 4;            // first window of pass 1: q-4 .. q+4
 constexpr int kNear2 = 2;            // first window of pass 2: q-2 .. q+2
 constexpr int kQB = 8;               // pass 1 outputs per register window
-constexpr int kPadTop = kNear1;      // pass 1 tile padding rows ("no site")
-constexpr int kPadBot = kNear1 + kQB;
 constexpr int kSqrtTab = 64;         // correctly rounded sqrt of 0..63 in shared memory
-constexpr int kMaxL0Smem = 256;      // pass 0 stages lines up to this length
-constexpr int kMaxL1 = 256;          // pass 1 tile: (L1 + 16) x 128 x 6 bytes
-constexpr int kMaxL2 = 4096;         // pass 2 line: (L + 8) x 8 + L x 2 bytes per warp
+constexpr int kMaxL1 = 1024;          // axis 1 of 3-D items: 32 staged columns (200 KB)
+constexpr int kMaxL2 = 4096;          // last axis: 8 staged rows (198 KB)
+constexpr int kShortLine = 128;       // rows up to this length are staged 32 at a time
+constexpr int kMediumLine = 512;      // longer rows take 512 threads per tile
 
 struct CompactParams {
     int ndim;        // 2 or 3
@@ -62,6 +50,8 @@ struct CompactParams {
     int64_t batch;
     int64_t numel;   // batch * numel_item
     int64_t numel_item;
+    uint32_t w0, w1, w2;  // squared voxel sizes of the axes in units of unit2 (1 for unit spacing)
+    float unit2;          // a power of 4
 };
 
 // floor(sqrt(u)) for 0 <= u < 2^31 (the float estimate is off by at most one).
@@ -106,581 +96,31 @@ __device__ __forceinline__ bool widen(int q, int L, GF G, uint32_t &best, int &b
     return true;
 }
 
-// ------------------------------------------------------------------ pass 0
-// Nearest background along axis 0, written as its position f0 (-1: none).
-// Staged variant: a block owns 128 adjacent columns of one item, 4 threads
-// per column, each sweeping a quarter of the column; the quarters exchange
-// their first/last background position through shared memory.
-template <typename In>
-__device__ __forceinline__ void edt_c0_smem_block(const int64_t blk, const In *__restrict__ in,
-                                                  int16_t *__restrict__ c1, const CompactParams &p) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int L = p.L0;
-    const int64_t inner = p.numel_item / L;
-    uint8_t *fg = smem_raw;                                              // [L][kCols]
-    int16_t *prev = reinterpret_cast<int16_t *>(smem_raw + L * kCols);   // [L][kCols]
-    int16_t *seg_last = prev + L * kCols;                                // [kSegs][kCols]
-    int16_t *seg_first = seg_last + kSegs * kCols;                       // [kSegs][kCols]
-    const int64_t cblocks = (inner + kCols - 1) / kCols;
-    const int64_t item = blk / cblocks;
-    const int64_t c0 = (blk - item * cblocks) * kCols;
-    const int64_t base = item * p.numel_item + c0;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // stage: 16 warps take rows w, w+16, ...; lane covers columns 4*lane .. 4*lane+3
-    for (int y0 = warp; y0 < L; y0 += 16 * 4) {
-        In v[4][4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int y = y0 + 16 * r;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int64_t c = c0 + 4 * lane + k;
-                v[r][k] = (y < L && c < inner) ? in[base + (int64_t)y * inner + 4 * lane + k] : (In)1;
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int y = y0 + 16 * r;
-            if (y < L) {
-                uint32_t word = 0;
-#pragma unroll
-                for (int k = 0; k < 4; k++) word |= (uint32_t)(v[r][k] != (In)0) << (8 * k);
-                reinterpret_cast<uint32_t *>(fg + y * kCols)[lane] = word;
-            }
-        }
-    }
-    __syncthreads();
-    const int col = tid % kCols, seg = tid / kCols;
-    const int S = (L + kSegs - 1) / kSegs;
-    const int ya = seg * S < L ? seg * S : L, yb = (seg + 1) * S < L ? (seg + 1) * S : L;
-    int last = -1, first = -1;
-    for (int y = ya; y < yb; y++) {
-        if (fg[y * kCols + col] == 0) {
-            last = y;
-            first = first < 0 ? y : first;
-        }
-        prev[y * kCols + col] = (int16_t)last;
-    }
-    seg_last[seg * kCols + col] = (int16_t)last;
-    seg_first[seg * kCols + col] = (int16_t)first;
-    __syncthreads();
-    int carry_prev = -1, next = -1;
-    for (int s = seg - 1; s >= 0 && carry_prev < 0; s--) carry_prev = seg_last[s * kCols + col];
-    for (int s = seg + 1; s < kSegs && next < 0; s++) next = seg_first[s * kCols + col];
-    if (c0 + col >= inner) return;
-    int16_t *out = c1 + base + col + (int64_t)(yb - 1) * inner;
-    for (int y = yb - 1; y >= ya; y--, out -= inner) {
-        int pv = prev[y * kCols + col];
-        if (pv < 0) pv = carry_prev;
-        if (pv == y) next = y;
-        const int f = (pv >= 0 && (next < 0 || y - pv <= next - y)) ? pv : next;
-        *out = (int16_t)f;
-    }
-}
-
-// Grid-stride over column blocks (one resident wave when per-item flags are
-// given, as for the fused passes).
-template <typename In>
-__global__ void __launch_bounds__(kCols *kSegs) edt_c0_smem_kernel(const In *__restrict__ in,
-                                                                   int16_t *__restrict__ c1, CompactParams p,
-                                                                   const int *__restrict__ todo) {
-    pdl_wait();  // launched after the shell search: its flags are complete
-    // the plane passes may be scheduled now: the flags they read are final
-    pdl_trigger();
-    const int64_t cblocks = (p.numel_item / p.L0 + kCols - 1) / kCols;
-    const int64_t nblk = p.batch * cblocks;
-    for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-        if (todo && !todo[blk / cblocks]) continue;  // item finished by the shell pass
-        edt_c0_smem_block<In>(blk, in, c1, p);
-        __syncthreads();  // the next block reuses shared memory
-    }
-}
-
-// Unstaged variant for long axis-0 lines: one thread per column, two sweeps
-// through global memory with 8 loads in flight.
-template <typename In>
-__global__ void __launch_bounds__(128) edt_c0_kernel(const In *__restrict__ in, int16_t *__restrict__ c1,
-                                                     CompactParams p) {
-    const int64_t inner = p.numel_item / p.L0;
-    const int64_t nlines = p.batch * inner;
-    const int64_t line = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (line >= nlines) return;
-    const int64_t item = line / inner;
-    const int64_t i = line - item * inner;
-    const int64_t base = item * p.numel_item + i;
-    const int L = p.L0;
-    int last = -1;
-    int q = 0;
-    for (; q + 8 <= L; q += 8) {
-        In v[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = in[base + (int64_t)(q + k) * inner];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            if (v[k] == (In)0) last = q + k;
-            c1[base + (int64_t)(q + k) * inner] = (int16_t)last;
-        }
-    }
-    for (; q < L; q++) {
-        if (in[base + (int64_t)q * inner] == (In)0) last = q;
-        c1[base + (int64_t)q * inner] = (int16_t)last;
-    }
-    int next = -1;
-    q = L - 1;
-    for (; q - 8 >= -1; q -= 8) {
-        int prv[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) prv[k] = c1[base + (int64_t)(q - k) * inner];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int z = q - k;
-            if (prv[k] == z) next = z;
-            const int f = (prv[k] >= 0 && (next < 0 || z - prv[k] <= next - z)) ? prv[k] : next;
-            c1[base + (int64_t)z * inner] = (int16_t)f;
-        }
-    }
-    for (; q >= 0; q--) {
-        const int pv = c1[base + (int64_t)q * inner];
-        if (pv == q) next = q;
-        const int f = (pv >= 0 && (next < 0 || q - pv <= next - q)) ? pv : next;
-        c1[base + (int64_t)q * inner] = (int16_t)f;
-    }
-}
-
-// ------------------------------------------------------------------ pass 1
-// 3-D only: lines along axis 1 at fixed (item, z, x).  A block owns the
-// (L1 x 128) tile of one (item, z) plane: shifted values gk = g << 5 and f0.
-// Output per voxel: packed (f0 | f1 << 16); f0 = -1 when no site.
-__global__ void __launch_bounds__(kCols *kSegs) edt_c1_kernel(const int16_t *__restrict__ c1,
-                                                              int32_t *__restrict__ c2,
-                                                              int16_t *__restrict__ gstack, CompactParams p) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int L0 = p.L0, L1 = p.L1, W = p.L2;
-    const int rows = L1 + kPadTop + kPadBot;
-    uint32_t *gk = reinterpret_cast<uint32_t *>(smem_raw) + kPadTop * kCols;  // rows -kPadTop .. L1+kPadBot-1
-    int16_t *f0t = reinterpret_cast<int16_t *>(smem_raw + (size_t)rows * kCols * 4) + kPadTop * kCols;
-    int *colflag = reinterpret_cast<int *>(smem_raw + (size_t)rows * kCols * 6);
-    const int xblocks = (W + kCols - 1) / kCols;
-    const int64_t item_z = blockIdx.x / xblocks;
-    const int xb = (int)(blockIdx.x - item_z * xblocks);
-    const int64_t item = item_z / L0;
-    const int z = (int)(item_z - item * L0);
-    const int x0 = xb * kCols;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t plane = item * p.numel_item + (int64_t)z * L1 * W;
-    for (int i = tid; i < (kPadTop + kPadBot) * kCols; i += kCols * kSegs) {
-        const int r = i / kCols, c = i % kCols;
-        const int y = r < kPadTop ? r - kPadTop : L1 + r - kPadTop;
-        gk[y * kCols + c] = kBig << kKeyShift;
-        f0t[y * kCols + c] = -1;
-    }
-    if (tid < kCols) colflag[tid] = 0;
-    // stage rows: 16 warps, 4 int16 per lane, 4 rows in flight per warp
-    const bool vec = (W % 4) == 0;
-    for (int y0 = warp; y0 < L1; y0 += 16 * 4) {
-        int16_t v[4][4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int y = y0 + 16 * r;
-            const int64_t rb = plane + (int64_t)y * W + x0 + 4 * lane;
-            if (y < L1 && vec && x0 + 4 * lane + 3 < W) {
-                const short4 s4 = *reinterpret_cast<const short4 *>(c1 + rb);
-                v[r][0] = s4.x;
-                v[r][1] = s4.y;
-                v[r][2] = s4.z;
-                v[r][3] = s4.w;
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    v[r][k] = (y < L1 && x0 + 4 * lane + k < W) ? c1[rb + k] : (int16_t)-1;
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int y = y0 + 16 * r;
-            if (y < L1) {
-                uint4 g4;
-                uint32_t *gp = &g4.x;
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const int f = v[r][k];
-                    gp[k] = (f < 0 ? kBig : (uint32_t)((z - f) * (z - f))) << kKeyShift;
-                }
-                *reinterpret_cast<uint4 *>(gk + y * kCols + 4 * lane) = g4;
-                short4 s4;
-                s4.x = v[r][0];
-                s4.y = v[r][1];
-                s4.z = v[r][2];
-                s4.w = v[r][3];
-                *reinterpret_cast<short4 *>(f0t + y * kCols + 4 * lane) = s4;
-            }
-        }
-    }
-    __syncthreads();
-    const int xl = tid % kCols, seg = tid / kCols;
-    const int x = x0 + xl;
-    const uint32_t *gcol = gk + xl;  // element y at gcol[y * kCols]
-    const int16_t *fcol = f0t + xl;
-    int32_t *out = c2 + plane + x;
-    auto G = [&](int pp) { return gcol[pp * kCols] >> kKeyShift; };
-    bool fallback = false;
-    if (x < W) {
-        const int qa = seg * L1 / kSegs, qb = (seg + 1) * L1 / kSegs;
-        constexpr int NW = kQB + 2 * kNear1;
-        for (int q0 = qa; q0 < qb && !fallback; q0 += kQB) {
-            uint32_t w[NW];
-#pragma unroll
-            for (int j = 0; j < NW; j++) w[j] = gcol[(q0 - kNear1 + j) * kCols];
-#pragma unroll
-            for (int i = 0; i < kQB; i++) {
-                const int q = q0 + i;
-                if (q < qb && !fallback) {
-                    const uint32_t key = window_key<kNear1>(w + i);
-                    uint32_t best = key >> kKeyShift;
-                    int bp = q - kNear1 + (int)(key & 31u);
-                    if (best >= (kNear1 + 1) * (kNear1 + 1) && !widen<kNear1>(q, L1, G, best, bp)) {
-                        fallback = true;
-                    } else {
-                        const int bf = fcol[bp * kCols];
-                        out[(int64_t)q * W] = best >= kBig ? -1 : ((int32_t)(uint16_t)bf | (bp << 16));
-                    }
-                }
-            }
-        }
-    }
-    if (fallback) colflag[xl] = 1;
-    __syncthreads();
-    if (seg != 0 || x >= W || !colflag[xl]) return;
-    // exact lower envelope of the whole line; stack in the workspace
-    const int64_t nlines = p.batch * (int64_t)L0 * W;
-    const int64_t lid = (item * L0 + z) * (int64_t)W + x;
-    int k = -1, top = 0, sec = 0;
-    int32_t Gtop = 0, Gsec = 0;
-    for (int q = 0; q < L1; q++) {
-        const uint32_t gq = G(q);
-        if (gq >= kBig) continue;
-        const int32_t Gq = (int32_t)gq + q * q;
-        while (k >= 1) {
-            const long long lhs = (long long)(Gq - Gtop) * (top - sec);
-            const long long rhs = (long long)(Gtop - Gsec) * (q - top);
-            if (lhs > rhs) break;
-            k--;
-            top = sec;
-            Gtop = Gsec;
-            if (k >= 1) {
-                sec = gstack[(int64_t)(k - 1) * nlines + lid];
-                Gsec = (int32_t)G(sec) + sec * sec;
-            }
-        }
-        k++;
-        gstack[(int64_t)k * nlines + lid] = (int16_t)q;
-        sec = top;
-        Gsec = Gtop;
-        top = q;
-        Gtop = Gq;
-    }
-    if (k < 0) {
-        for (int q = 0; q < L1; q++) out[(int64_t)q * W] = -1;
-        return;
-    }
-    int j = 0;
-    int cur = gstack[lid];
-    uint32_t gcur = G(cur);
-    int nxt = 0;
-    uint32_t gnxt = 0;
-    if (k >= 1) {
-        nxt = gstack[nlines + lid];
-        gnxt = G(nxt);
-    }
-    for (int q = 0; q < L1; q++) {
-        uint32_t fc = (uint32_t)((q - cur) * (q - cur)) + gcur;
-        while (j < k) {
-            const uint32_t fn = (uint32_t)((q - nxt) * (q - nxt)) + gnxt;
-            if (!(fn < fc)) break;
-            j++;
-            cur = nxt;
-            gcur = gnxt;
-            fc = fn;
-            if (j < k) {
-                nxt = gstack[(int64_t)(j + 1) * nlines + lid];
-                gnxt = G(nxt);
-            }
-        }
-        out[(int64_t)q * W] = (int32_t)(uint16_t)fcol[cur * kCols] | (cur << 16);
-    }
-}
-
-// ------------------------------------------------------------------ pass 2
 __device__ __forceinline__ float dist_of(uint32_t best, const float *tab) {
     if (best < kSqrtTab) return tab[best];
     return best < (1u << 24) ? __fsqrt_rn((float)best) : (float)sqrt((double)best);
 }
 
-// Last axis, one warp per line.  IN3D: input is packed (f0, f1) per voxel;
-// otherwise (2-D) it is f0.  VEC (lines a multiple of 128 long): each lane
-// owns 4 consecutive voxels of every 128-voxel chunk, loads them with one
-// vector load and writes each output plane with one 16-byte store.
-template <bool IN3D, bool VEC>
-__global__ void __launch_bounds__(kC2Warps * 32) edt_c2_kernel(const void *__restrict__ cin, float *__restrict__ dist,
-                                                               int32_t *__restrict__ indices,
-                                                               int32_t *__restrict__ sqdist, CompactParams p,
-                                                               int warps) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int L = IN3D ? p.L2 : p.L1;
-    const int Lp = L + 8;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float *tab = reinterpret_cast<float *>(smem_raw);                              // sqrt table
-    uint32_t *base_u = reinterpret_cast<uint32_t *>(smem_raw) + kSqrtTab;
-    uint32_t *sg = base_u + warp * Lp + 4;                                         // g << 5, padded by 4
-    int32_t *sf = reinterpret_cast<int32_t *>(base_u) + (warps + warp) * Lp + 4;   // packed feature
-    int16_t *st = reinterpret_cast<int16_t *>(base_u + 2 * warps * Lp) + warp * L;  // envelope stack
-    for (int i = threadIdx.x; i < kSqrtTab; i += blockDim.x) tab[i] = __fsqrt_rn((float)i);
-    __syncthreads();
-    const int64_t lines_per_item = IN3D ? (int64_t)p.L0 * p.L1 : (int64_t)p.L0;
-    const int64_t nlines = p.batch * lines_per_item;
-    const int64_t line = (int64_t)blockIdx.x * warps + warp;
-    if (line >= nlines) return;
-    const int64_t item = line / lines_per_item;
-    const int64_t rem = line - item * lines_per_item;
-    int z = 0, y;
-    if (IN3D) {
-        z = (int)(rem / p.L1);
-        y = (int)(rem - (int64_t)z * p.L1);
-    } else {
-        y = (int)rem;
-    }
-    const int64_t base = line * L;
-    if (lane < 8) {
-        const int q = lane < 4 ? lane - 4 : L + lane - 4;
-        sg[q] = kBig << kKeyShift;
-        sf[q] = -1;
-    }
-    auto gval = [&](int32_t f) -> uint32_t {
-        if (IN3D) {
-            const int f0 = (int16_t)(f & 0xffff), f1 = f >> 16;
-            return f0 < 0 ? kBig : (uint32_t)((z - f0) * (z - f0) + (y - f1) * (y - f1));
-        }
-        return f < 0 ? kBig : (uint32_t)((y - f) * (y - f));
-    };
-    // stage the line
-    bool any = false;
-    if (VEC) {
-        for (int c = 0; c < L; c += 128) {
-            const int q0 = c + 4 * lane;
-            int32_t f[4];
-            if (IN3D) {
-                const int4 v = *reinterpret_cast<const int4 *>(reinterpret_cast<const int32_t *>(cin) + base + q0);
-                f[0] = v.x;
-                f[1] = v.y;
-                f[2] = v.z;
-                f[3] = v.w;
-            } else {
-                const short4 v = *reinterpret_cast<const short4 *>(reinterpret_cast<const int16_t *>(cin) + base + q0);
-                f[0] = v.x;
-                f[1] = v.y;
-                f[2] = v.z;
-                f[3] = v.w;
-            }
-            uint4 g4;
-            g4.x = gval(f[0]);
-            g4.y = gval(f[1]);
-            g4.z = gval(f[2]);
-            g4.w = gval(f[3]);
-            any |= (g4.x < kBig) | (g4.y < kBig) | (g4.z < kBig) | (g4.w < kBig);
-            g4.x <<= kKeyShift;
-            g4.y <<= kKeyShift;
-            g4.z <<= kKeyShift;
-            g4.w <<= kKeyShift;
-            *reinterpret_cast<uint4 *>(sg + q0) = g4;
-            *reinterpret_cast<int4 *>(sf + q0) = make_int4(f[0], f[1], f[2], f[3]);
-        }
-    } else {
-        for (int q0 = lane; q0 < L; q0 += 128) {
-            int32_t fv[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int q = q0 + 32 * k;
-                if (IN3D)
-                    fv[k] = q < L ? reinterpret_cast<const int32_t *>(cin)[base + q] : -1;
-                else
-                    fv[k] = q < L ? (int32_t)reinterpret_cast<const int16_t *>(cin)[base + q] : -1;
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int q = q0 + 32 * k;
-                if (q < L) {
-                    const uint32_t g = gval(fv[k]);
-                    sg[q] = g << kKeyShift;
-                    sf[q] = fv[k];
-                    any |= g < kBig;
-                }
-            }
-        }
-    }
-    any = __any_sync(0xffffffffu, any);
-    __syncwarp();
-    const int64_t numel = p.numel;
-    if (!any) {
-        // no background anywhere in the item: virtual site (-1, 0, ...)
-        for (int q = lane; q < L; q += 32) {
-            const int64_t gi = base + q;
-            const uint32_t s2 = IN3D ? (uint32_t)((z + 1) * (z + 1) + y * y + q * q)
-                                     : (uint32_t)((y + 1) * (y + 1) + q * q);
-            if (dist) dist[gi] = dist_of(s2, tab);
-            if (sqdist) sqdist[gi] = (int32_t)s2;
-            if (indices) {
-                indices[gi] = -1;
-                indices[numel + gi] = 0;
-                if (IN3D) indices[2 * numel + gi] = 0;
-            }
-        }
-        return;
-    }
-    auto G = [&](int pp) { return sg[pp] >> kKeyShift; };
-    bool fallback = false;
-    if (VEC) {
-        for (int c = 0; c < L && !fallback; c += 128) {
-            const int q0 = c + 4 * lane;
-            uint32_t w[12];  // shifted g at q0-4 .. q0+7
-            const uint4 a = *reinterpret_cast<const uint4 *>(sg + q0 - 4);
-            const uint4 b = *reinterpret_cast<const uint4 *>(sg + q0);
-            const uint4 d4 = *reinterpret_cast<const uint4 *>(sg + q0 + 4);
-            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-            w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-            w[8] = d4.x; w[9] = d4.y; w[10] = d4.z; w[11] = d4.w;
-            float dv[4];
-            int32_t i0[4], i1[4], i2[4], sq[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int q = q0 + i;
-                const uint32_t key = window_key<kNear2>(w + i + 2);
-                uint32_t best = key >> kKeyShift;
-                int bp = q - kNear2 + (int)(key & 31u);
-                if (best >= (kNear2 + 1) * (kNear2 + 1) && !widen<kNear2>(q, L, G, best, bp)) fallback = true;
-                const int32_t f = sf[bp];
-                dv[i] = dist_of(best, tab);
-                sq[i] = (int32_t)best;
-                if (IN3D) {
-                    i0[i] = (int16_t)(f & 0xffff);
-                    i1[i] = f >> 16;
-                    i2[i] = bp;
-                } else {
-                    i0[i] = f;
-                    i1[i] = bp;
-                }
-            }
-            if (fallback) break;
-            const int64_t gi = base + q0;
-            if (dist) *reinterpret_cast<float4 *>(dist + gi) = make_float4(dv[0], dv[1], dv[2], dv[3]);
-            if (sqdist) *reinterpret_cast<int4 *>(sqdist + gi) = make_int4(sq[0], sq[1], sq[2], sq[3]);
-            if (indices) {
-                *reinterpret_cast<int4 *>(indices + gi) = make_int4(i0[0], i0[1], i0[2], i0[3]);
-                *reinterpret_cast<int4 *>(indices + numel + gi) = make_int4(i1[0], i1[1], i1[2], i1[3]);
-                if (IN3D)
-                    *reinterpret_cast<int4 *>(indices + 2 * numel + gi) = make_int4(i2[0], i2[1], i2[2], i2[3]);
-            }
-        }
-    } else {
-        for (int q = lane; q < L; q += 32) {
-            uint32_t w[2 * kNear2 + 1];
-#pragma unroll
-            for (int k = 0; k <= 2 * kNear2; k++) w[k] = sg[q - kNear2 + k];
-            const uint32_t key = window_key<kNear2>(w);
-            uint32_t best = key >> kKeyShift;
-            int bp = q - kNear2 + (int)(key & 31u);
-            if (best >= (kNear2 + 1) * (kNear2 + 1) && !widen<kNear2>(q, L, G, best, bp)) {
-                fallback = true;
-                break;
-            }
-            const int64_t gi = base + q;
-            const int32_t f = sf[bp];
-            if (dist) dist[gi] = dist_of(best, tab);
-            if (sqdist) sqdist[gi] = (int32_t)best;
-            if (indices) {
-                if (IN3D) {
-                    indices[gi] = (int16_t)(f & 0xffff);
-                    indices[numel + gi] = f >> 16;
-                    indices[2 * numel + gi] = bp;
-                } else {
-                    indices[gi] = f;
-                    indices[numel + gi] = bp;
-                }
-            }
-        }
-    }
-    if (!__any_sync(0xffffffffu, fallback)) return;
-    // exact lower envelope: lane 0 builds it into the shared stack, every
-    // lane then locates its positions by binary search
-    int ktop = 0;
-    if (lane == 0) {
-        int k = -1, top = 0, sec = 0;
-        int32_t Gtop = 0, Gsec = 0;
-        for (int q = 0; q < L; q++) {
-            const uint32_t gq = G(q);
-            if (gq >= kBig) continue;
-            const int32_t Gq = (int32_t)gq + q * q;
-            while (k >= 1) {
-                const long long lhs = (long long)(Gq - Gtop) * (top - sec);
-                const long long rhs = (long long)(Gtop - Gsec) * (q - top);
-                if (lhs > rhs) break;
-                k--;
-                top = sec;
-                Gtop = Gsec;
-                if (k >= 1) {
-                    sec = st[k - 1];
-                    Gsec = (int32_t)G(sec) + sec * sec;
-                }
-            }
-            st[++k] = (int16_t)q;
-            sec = top;
-            Gsec = Gtop;
-            top = q;
-            Gtop = Gq;
-        }
-        ktop = k;
-    }
-    ktop = __shfl_sync(0xffffffffu, ktop, 0);
-    __syncwarp();
-    for (int q = lane; q < L; q += 32) {
-        // largest k with f_{v[k]}(q) < f_{v[k-1]}(q): the envelope segment of q
-        int lo = 0, hi = ktop;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            const int a = st[mid - 1], b = st[mid];
-            const uint32_t fa = (uint32_t)((q - a) * (q - a)) + G(a);
-            const uint32_t fb = (uint32_t)((q - b) * (q - b)) + G(b);
-            if (fb < fa)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        const int bp = st[lo];
-        const uint32_t best = (uint32_t)((q - bp) * (q - bp)) + G(bp);
-        const int64_t gi = base + q;
-        const int32_t f = sf[bp];
-        if (dist) dist[gi] = dist_of(best, tab);
-        if (sqdist) sqdist[gi] = (int32_t)best;
-        if (indices) {
-            if (IN3D) {
-                indices[gi] = (int16_t)(f & 0xffff);
-                indices[numel + gi] = f >> 16;
-                indices[2 * numel + gi] = bp;
-            } else {
-                indices[gi] = f;
-                indices[numel + gi] = bp;
-            }
-        }
-    }
+// Distance of v units of 4^-k (unit2 = 4^-k): float(v) is exact below 2^24 and so is its
+// product with a power of two, and a correctly rounded float sqrt of an exact input
+// equals the rounded float64 sqrt.
+__device__ __forceinline__ float line_dist(uint32_t v, float unit2) {
+    // (a square root of zero would leave the fast path of __fsqrt_rn)
+    const float d = v < (1u << 24) ? __fsqrt_rn((float)max(v, 1u) * unit2) : (float)sqrt((double)v * (double)unit2);
+    return v ? d : 0.0f;
 }
 
+#include "edt_lines.cuh"
+
 // ------------------------------------------------------ passes 1 + 2 fused
-// 3-D items with L0, L1 <= 255 and L2 a multiple of 4: one CTA per (item, z)
-// plane runs pass 1 (axis 1) and pass 2 (axis 2) back to back on chip.  The
+// Planes of ragged batches: one CTA per (item, z) plane with sizes up to 180
+// runs pass 1 (axis 1) and pass 2 (axis 2) back to back on chip.  The
 // plane's pass-0 features are staged as bytes (f0, 255 = none); pass 1
 // writes packed (f0 | f1 << 8) uint16 features (0xFFFF = none) to a second
 // shared-memory plane, which pass 2 reads row by row; only the final
-// outputs go to global memory.  Same windows, widening, tie rules and
-// envelope fallbacks as edt_c1_kernel / edt_c2_kernel.
+// outputs go to global memory.  A window of candidates first (exact when its
+// best value is below (K + 1)^2), widened to the exact radius, then the exact
+// lower envelope of the line.
 constexpr int kC12Threads = 256;
 constexpr int kC12Warps = kC12Threads / 32;
 constexpr int kC12Cols = 128;  // pass-1 columns per group (2 threads per column)
@@ -728,10 +168,8 @@ __host__ __device__ inline C12Smem c12_smem(int L1, int L2) {
 
 // One (L1 x W) plane of the fused passes 1 + 2: the plane's pass-0 features
 // start at c1 + plane and its outputs at plane in each output (index planes
-// `numel` apart); z is the plane's axis-0 coordinate.  VEC: W % 4 == 0 and
-// 16-byte aligned planes (8-byte loads, 16-byte stores); otherwise every
-// access is scalar, for items packed at any offset.
-template <bool VEC>
+// `numel` apart); z is the plane's axis-0 coordinate.  Every access is scalar:
+// items are packed at any offset.
 __device__ __forceinline__ void edt_c12_plane(const int64_t plane, const int z, const int L1, const int W,
                                               const int64_t numel, const int16_t *__restrict__ c1,
                                               float *__restrict__ dist, int32_t *__restrict__ indices,
@@ -757,21 +195,11 @@ __device__ __forceinline__ void edt_c12_plane(const int64_t plane, const int z, 
         const int y = i / (kC12PadX + padr), k = i % (kC12PadX + padr);
         p1[y * rowp + (k < kC12PadX ? k : kC12PadX + W + (k - kC12PadX))] = kNoF01;
     }
-    if (VEC) {  // stage the pass-0 features of the plane as bytes, 4 per lane per row
-        for (int i = tid; i < L1 * (W / 4); i += kC12Threads) {
-            const int y = i / (W / 4), c4 = i % (W / 4);
-            const short4 v = *reinterpret_cast<const short4 *>(c1 + plane + (int64_t)y * W + 4 * c4);
-            const uint32_t b0 = v.x < 0 ? kNoF0 : (uint32_t)v.x, b1 = v.y < 0 ? kNoF0 : (uint32_t)v.y;
-            const uint32_t b2 = v.z < 0 ? kNoF0 : (uint32_t)v.z, b3 = v.w < 0 ? kNoF0 : (uint32_t)v.w;
-            reinterpret_cast<uint32_t *>(f0s + y * W)[c4] = b0 | (b1 << 8) | (b2 << 16) | (b3 << 24);
-        }
-    } else {
-        // (L2 loads: in the ragged launch other SMs wrote these features after
-        // a grid barrier, so no L1 line may serve them)
-        for (int i = tid; i < L1 * W; i += kC12Threads) {
-            const int16_t v = __ldcg(c1 + plane + i);
-            f0s[i] = v < 0 ? kNoF0 : (uint8_t)v;
-        }
+    // (L2 loads: other SMs wrote these features before a grid barrier, so no L1
+    // line may serve them)
+    for (int i = tid; i < L1 * W; i += kC12Threads) {
+        const int16_t v = __ldcg(c1 + plane + i);
+        f0s[i] = v < 0 ? kNoF0 : (uint8_t)v;
     }
     __syncthreads();
 
@@ -924,8 +352,7 @@ __device__ __forceinline__ void edt_c12_plane(const int64_t plane, const int z, 
                 const uint32_t key = window_key<kNear2>(w + i + 2);
                 uint32_t best = key >> kKeyShift;
                 int bp = q - kNear2 + (int)(key & 31u);
-                // (VEC: q < W always; otherwise the round-up positions have no site
-                // and are neither searched nor written)
+                // (the round-up positions have no site and are neither searched nor written)
                 if (q < W && best >= (kNear2 + 1) * (kNear2 + 1) && !widen<kNear2>(q, W, G2, best, bp, kC12Far))
                     fallback = true;
                 const uint32_t f = row[bp];
@@ -937,25 +364,15 @@ __device__ __forceinline__ void edt_c12_plane(const int64_t plane, const int z, 
             }
             if (fallback) break;
             const int64_t gi = base + q0;
-            if (VEC) {
-                if (dist) *reinterpret_cast<float4 *>(dist + gi) = make_float4(dv[0], dv[1], dv[2], dv[3]);
-                if (sqdist) *reinterpret_cast<int4 *>(sqdist + gi) = make_int4(sq[0], sq[1], sq[2], sq[3]);
-                if (indices) {
-                    *reinterpret_cast<int4 *>(indices + gi) = make_int4(i0[0], i0[1], i0[2], i0[3]);
-                    *reinterpret_cast<int4 *>(indices + numel + gi) = make_int4(i1[0], i1[1], i1[2], i1[3]);
-                    *reinterpret_cast<int4 *>(indices + 2 * numel + gi) = make_int4(i2[0], i2[1], i2[2], i2[3]);
-                }
-            } else {
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if (q0 + i >= W) break;
-                    if (dist) dist[gi + i] = dv[i];
-                    if (sqdist) sqdist[gi + i] = sq[i];
-                    if (indices) {
-                        indices[gi + i] = i0[i];
-                        indices[numel + gi + i] = i1[i];
-                        indices[2 * numel + gi + i] = i2[i];
-                    }
+            for (int i = 0; i < 4; i++) {
+                if (q0 + i >= W) break;
+                if (dist) dist[gi + i] = dv[i];
+                if (sqdist) sqdist[gi + i] = sq[i];
+                if (indices) {
+                    indices[gi + i] = i0[i];
+                    indices[numel + gi + i] = i1[i];
+                    indices[2 * numel + gi + i] = i2[i];
                 }
             }
         }
@@ -1044,32 +461,6 @@ __device__ __forceinline__ void edt_c12_plane(const int64_t plane, const int z, 
     }
 }
 
-// Grid-stride over planes: with per-item flags (after the shell search) the
-// grid is one resident wave, so items the search finished cost one flag
-// read per plane.
-__global__ void __launch_bounds__(kC12Threads, 3) edt_c12_kernel(const int16_t *__restrict__ c1, float *__restrict__ dist,
-                                                              int32_t *__restrict__ indices,
-                                                              int32_t *__restrict__ sqdist, CompactParams p,
-                                                              const int *__restrict__ todo) {
-    // Launched behind pass 0, which lets this grid be scheduled once the shell
-    // search has completed: the flags are final here (read through L2), and a
-    // block waits for pass 0's features only when it has a plane to compute.
-    const int64_t nblk = p.batch * (int64_t)p.L0;
-    bool waited = false;
-    for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-        const int64_t item = blk / p.L0;
-        if (todo && !__ldcg(todo + item)) continue;  // item finished by the shell pass
-        if (!waited) {
-            pdl_wait();  // pass 0's features are complete
-            waited = true;
-        }
-        const int z = (int)(blk - item * p.L0);
-        edt_c12_plane<true>(item * p.numel_item + (int64_t)z * p.L1 * p.L2, z, p.L1, p.L2, p.numel, c1, dist, indices,
-                            sqdist);
-        __syncthreads();  // the next plane reuses shared memory
-    }
-}
-
 // ------------------------------------------- ragged batches of 3-D items
 // The fused plane passes over a ragged batch (items packed at any offset,
 // every axis at most kRaggedC12MaxLine): one cooperative launch whose first
@@ -1155,7 +546,7 @@ __global__ void __launch_bounds__(kC12Threads, 2) ragged_edt3_kernel(RaggedC12Ar
         }
         const ReItem &it = items[lo];
         const int z = (int)(k - it.plane_begin), H = it.shape[1], W = it.shape[2];
-        edt_c12_plane<false>(it.off + (int64_t)z * H * W, z, H, W, A.total, A.c1, A.dist, A.indices, A.sqdist);
+        edt_c12_plane(it.off + (int64_t)z * H * W, z, H, W, A.total, A.c1, A.dist, A.indices, A.sqdist);
         __syncthreads();  // the next plane reuses shared memory
     }
 }
@@ -1297,6 +688,8 @@ __global__ void __launch_bounds__(kShellThreads) edt_shell_kernel(const uint32_t
     const int nrows = min(kShellRows, L1 - y0);
     const int ww = sm.ww, pitch = sm.pitch, planep = sm.planep;
     const int tid = threadIdx.x;
+    // (marked already: the separable passes write the whole item)
+    const int marked = tid == 0 ? __ldcg(todo + item) : 0;
     if (tid == 0) s_unresolved = 0;
     for (int t = tid; t < kShellN; t += kShellThreads) {
         const uint32_t e = c_shell.v[t];
@@ -1328,7 +721,7 @@ __global__ void __launch_bounds__(kShellThreads) edt_shell_kernel(const uint32_t
             for (int c = 0; c < ww; c++) dst[kShellPadW + c] = in_item ? src[c] : 0u;
         }
     }
-    __syncthreads();
+    if (__syncthreads_or(marked)) return;
     // search: one 32-voxel word per thread
     const uint32_t *center = bits + kShellR * planep + kShellR * pitch + kShellPadW;  // (z, y0, word 0)
     for (int e = tid; e < nrows * ww; e += kShellThreads) {
@@ -1577,6 +970,7 @@ __global__ void __launch_bounds__(kShellCtThreads) edt_shell_ct_kernel(const uin
         // offset is the batch's i-th (earlier offsets keep priority), then
         // planes 0-2 take the bits of i and planes 3-8 the batch number.
         uint32_t U = 0u;
+        bool hopeless = false;
         {
             const int r = lane >> 2, wi = lane & 3;
             const int nb = min(32, W - 32 * wi);
@@ -1590,6 +984,15 @@ __global__ void __launch_bounds__(kShellCtThreads) edt_shell_ct_kernel(const uin
 #pragma unroll
             for (int t0 = 0; t0 < kShellN; t0 += kB) {
                 if (U == 0u) break;
+                // inside large objects most voxels stay open: leave early.  A background dense
+                // enough to end with kFarPerUnit open voxels (p^257 = 1/32) has p^t open after t
+                if (t0 == 24 || t0 == 64 || t0 == 128) {
+                    const int most = t0 == 24 ? 900 : (t0 == 64 ? 600 : 256);
+                    if ((int)__reduce_add_sync(__activemask(), (unsigned)__popc(U)) > most) {
+                        hopeless = true;
+                        break;
+                    }
+                }
                 uint32_t bg[kB];
                 uint32_t any = 0;
 #pragma unroll
@@ -1628,7 +1031,7 @@ __global__ void __launch_bounds__(kShellCtThreads) edt_shell_ct_kernel(const uin
             pw[2] = make_uint4(P[8], 0u, 0u, 0u);
         }
         const unsigned nfar = __reduce_add_sync(~0u, (unsigned)__popc(U));  // voxels beyond the shell
-        if (nfar > kFarPerUnit) {  // many: the item takes the separable passes
+        if (nfar > kFarPerUnit || __any_sync(~0u, hopeless)) {  // many: the item takes the separable passes
             if (lane == 0) atomicExch(&todo[item], 1);
             continue;
         }
@@ -2127,38 +1530,138 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace
 
-bool edt_compact_eligible(const Geometry &g, bool unit) {
-    if (!unit || (g.ndim != 2 && g.ndim != 3)) return false;
+// Spacings that are binary fractions n_d / 2^k with squared distances below 2^24 units of
+// 4^-k (1, 0.5, 2.5, 0.75 ...): every value of the float passes is then exact, and so the
+// integer passes give the same features and distances.
+bool edt_spacing(int ndim, const float *sampling, EdtSpacing *out) {
+    EdtSpacing s;
+    s.scaled = false;
+    s.unit2 = 1.0f;
+    for (int d = 0; d < 3; d++) s.w[d] = 1;
+    if (sampling) {
+        int k = 0;
+        for (; k <= 8; k++) {
+            bool whole = true;
+            for (int d = 0; d < ndim; d++) {
+                const double n = std::ldexp((double)sampling[d], k);
+                whole = whole && n == std::floor(n) && n >= 1.0 && n * n <= (double)kMaxWeight;
+            }
+            if (whole) break;
+        }
+        if (k > 8 || ndim > 3) return false;
+        for (int d = 0; d < ndim; d++) {
+            const int n = (int)std::ldexp((double)sampling[d], k);
+            s.w[d] = (uint32_t)(n * n);
+            s.scaled = s.scaled || sampling[d] != 1.0f;
+        }
+        s.unit2 = (float)std::ldexp(1.0, -2 * k);
+    }
+    *out = s;
+    return true;
+}
+
+bool edt_compact_eligible(const Geometry &g, const float *sampling, EdtSpacing *spacing) {
+    EdtSpacing sp;
+    if ((g.ndim != 2 && g.ndim != 3) || !edt_spacing(g.ndim, sampling, &sp)) return false;
+    if (spacing) *spacing = sp;
     int64_t sum = 0;
     for (int d = 0; d < g.ndim; d++) {
         if (g.shape[d] > 32767) return false;
-        sum += (g.shape[d] + 1) * (g.shape[d] + 1);
+        sum += (g.shape[d] + 1) * (g.shape[d] + 1) * (int64_t)sp.w[d];
     }
-    if (sum + 64 >= (int64_t)kBig) return false;  // every squared distance stays below kBig
+    // every squared distance stays below kBig (and, with a scale, exact in float)
+    if (sum + 64 >= (sp.scaled ? (int64_t)1 << 24 : (int64_t)kBig)) return false;
     if (g.ndim == 3 && g.shape[1] > kMaxL1) return false;
     if (g.shape[g.ndim - 1] > kMaxL2) return false;
     if (g.numel >= ((int64_t)1 << 40)) return false;
     return true;
 }
 
-// CTAs of one kernel resident at once on the device (one wave), at least one.
+// CTAs of one kernel resident at once on the device (one wave), at least one.  The last
+// answer of each kernel type and thread is kept (kernels are told apart by address).
 template <typename K>
 int64_t wave_ctas(K kernel, int threads, size_t smem) {
+    struct Last {
+        const void *fn;
+        int dev, threads;
+        size_t smem;
+        int64_t ctas;
+    };
+    static thread_local Last last[4] = {};
+    static thread_local int turn = 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    for (const Last &l : last)
+        if (l.fn == (const void *)kernel && l.dev == dev && l.threads == threads && l.smem == smem) return l.ctas;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
+    last[turn] = Last{(const void *)kernel, dev, threads, smem, (int64_t)per_sm * sm_count()};
+    turn = (turn + 1) & 3;
     return (int64_t)per_sm * sm_count();
 }
 
 size_t edt_compact_workspace(const Geometry &g) {
     const size_t n = (size_t)g.numel;
     size_t s = align256(n * 2);                               // f0 per voxel
-    if (g.ndim == 3) s += align256(n * 4) + align256(n * 2);  // (f0, f1) + pass-1 envelope stacks
+    if (g.ndim == 3) s += align256(n * 4) + align256(n * 2);  // (f0, f1), the shell search's flags
     return s;
 }
 
-int edt_compact_run(const void *input, int in_dtype, const Geometry &g, float *dist, int32_t *indices,
-                    int32_t *sqdist, unsigned char *ws, cudaStream_t stream) {
+namespace {
+
+// One pass over the lines: a resident wave striding over the tiles where items may be
+// finished already (todo), else a CTA per tile.
+template <int MODE, int NL, int T, int OUT>
+int launch_lines(const void *src, int32_t *c2, float *dist, int32_t *indices, int32_t *sqdist, const CompactParams &p,
+                 const int *todo, cudaStream_t stream) {
+    const int L = MODE == 2 ? p.L2 : p.L1;
+    const int64_t rows = MODE == 0 ? p.L0 : (int64_t)p.L0 * p.L1;
+    const int64_t tiles = p.batch * (MODE == 1 ? (int64_t)p.L0 * ceil_div(p.L2, NL) : ceil_div(rows, NL));
+    if (tiles >= ((int64_t)1 << 31)) return fail(TM_ERR_TOO_LARGE, "too many blocks");
+    const size_t smem = line_tile(NL, L).total;
+    if (smem > 48 * 1024)
+        TM_CHECK_CUDA(cudaFuncSetAttribute(edt_line_kernel<MODE, NL, T, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem));
+    const int64_t grid = todo ? std::min<int64_t>(tiles, wave_ctas(edt_line_kernel<MODE, NL, T, OUT>, T, smem)) : tiles;
+    TM_CHECK_CUDA(launch_pdl(edt_line_kernel<MODE, NL, T, OUT>, dim3((unsigned)grid), dim3(T), smem, stream, src, c2,
+                             dist, indices, sqdist, p, todo));
+    TM_LAUNCH_CHECK("edt_line_kernel");
+    return TM_OK;
+}
+
+template <typename In>
+int launch_bits0(const In *in, int16_t *c1, const CompactParams &p, const int *todo, cudaStream_t stream) {
+    const int64_t inner = p.numel_item / p.L0;
+    const int nw = (p.L0 + 31) / 32, wpc = std::min(nw, kBitsWarps);
+    // 4 columns per lane once they fill the device (a warp per 32 rows and 128 columns)
+    const bool wide = inner % 4 == 0 && ((uintptr_t)in & (4 * sizeof(In) - 1)) == 0 &&
+                      p.batch * (inner / 128) * nw >= (int64_t)sm_count() * 32;
+    const int cols = wide ? 128 : 32;
+    const int groups = (int)std::max<int64_t>(1, std::min<int64_t>(kBitsWarps / wpc, ceil_div(inner, cols)));
+    const int64_t blocks = p.batch * ceil_div(inner, (int64_t)cols * groups);
+    if (blocks >= ((int64_t)1 << 31)) return fail(TM_ERR_TOO_LARGE, "too many blocks");
+    const dim3 threads(32 * wpc, groups);
+    const size_t smem = (size_t)nw * cols * groups * 4;
+    auto go = [&](auto kernel) -> int {
+        if (smem > 48 * 1024)
+            TM_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (todo) {  // overlaps the shell search's last CTAs
+            const int64_t grid = std::min<int64_t>(blocks, wave_ctas(kernel, 32 * wpc * groups, smem));
+            TM_CHECK_CUDA(launch_pdl(kernel, dim3((unsigned)grid), threads, smem, stream, in, c1, p, todo));
+        } else {
+            kernel<<<(unsigned)blocks, threads, smem, stream>>>(in, c1, p, todo);
+        }
+        TM_LAUNCH_CHECK("edt_bits0_kernel");
+        return TM_OK;
+    };
+    return wide ? go(edt_bits0_kernel<In, 4>) : go(edt_bits0_kernel<In, 1>);
+}
+
+}  // namespace
+
+int edt_compact_run(const void *input, int in_dtype, const Geometry &g, const EdtSpacing &spacing, float *dist,
+                    int32_t *indices, int32_t *sqdist, unsigned char *ws, cudaStream_t stream) {
     CompactParams p;
     std::memset(&p, 0, sizeof(p));
     p.ndim = g.ndim;
@@ -2168,25 +1671,30 @@ int edt_compact_run(const void *input, int in_dtype, const Geometry &g, float *d
     p.batch = g.batch;
     p.numel = g.numel;
     p.numel_item = g.numel_item;
+    p.w0 = spacing.w[0];
+    p.w1 = spacing.w[1];
+    p.w2 = spacing.w[2];
+    p.unit2 = spacing.unit2;
     const size_t n = (size_t)g.numel;
     int16_t *c1 = reinterpret_cast<int16_t *>(ws);
     int32_t *c2 = g.ndim == 3 ? reinterpret_cast<int32_t *>(ws + align256(n * 2)) : nullptr;
-    int16_t *stack1 = g.ndim == 3 ? reinterpret_cast<int16_t *>(ws + align256(n * 2) + align256(n * 4)) : nullptr;
-    const bool fused = g.ndim == 3 && p.L0 <= 254 && p.L1 <= 254 && (p.L2 % 4) == 0 && ((uintptr_t)dist & 15) == 0 &&
-                       ((uintptr_t)indices & 15) == 0 && ((uintptr_t)sqdist & 15) == 0 && (g.numel % 4) == 0 &&
-                       c12_smem(p.L1, p.L2).total <= 200 * 1024;
+    const bool shell_shape = g.ndim == 3 && !spacing.scaled && p.L0 <= 254 && p.L1 <= 254 && (p.L2 % 4) == 0 &&
+                             ((uintptr_t)dist & 15) == 0 && ((uintptr_t)indices & 15) == 0 &&
+                             ((uintptr_t)sqdist & 15) == 0 && (g.numel % 4) == 0 &&
+                             c12_smem(p.L1, p.L2).total <= 200 * 1024;
     // dense backgrounds: shell search first; the separable passes then run only
-    // for the items it could not finish (todo flags).  The (f0, f1) plane of
-    // the unfused pass 1 is unused on this path and holds the bitmap + flags.
+    // for the items it could not finish.  The (f0, f1) plane holds the bitmap
+    // until pass 1 writes it; the flags (todo) have the region behind it (rows are
+    // multiples of 4 voxels here, so 2 bytes a voxel hold 4 per item).
     int *todo = nullptr;
     // autotuned variant 1: the separable passes for every item (no shell search)
     const bool shell = tune_variant(kTuneEdt3D, tune_class(kTuneEdt3D, g.numel, 0)) != 1;
-    if (fused && p.L2 <= 1024 && shell) {
+    if (shell_shape && p.L2 <= 1024 && shell) {
         int st = TM_OK;
         const int ww = (p.L2 + 31) / 32;
         const int64_t nwords = g.batch * (int64_t)p.L0 * p.L1 * ww;
         uint32_t *bm = reinterpret_cast<uint32_t *>(c2);
-        todo = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(c2) + align256((size_t)nwords * 4));
+        todo = reinterpret_cast<int *>(ws + align256(n * 2) + align256(n * 4));
         // per-item flags, then (8-byte aligned) the shell kernel's 64-bit work
         // counter: zeroed by the bitmap kernel
         const int nclear = (int)((g.batch + 1) & ~(int64_t)1) + 2;
@@ -2236,100 +1744,26 @@ int edt_compact_run(const void *input, int in_dtype, const Geometry &g, float *d
         }
         TM_LAUNCH_CHECK("edt_shell_kernel");
     }
-    // pass 0
-    const int64_t inner0 = g.numel_item / g.shape[0];
-    if (p.L0 <= kMaxL0Smem) {
-        const int64_t blocks = g.batch * ceil_div(inner0, kCols);
-        if (blocks >= ((int64_t)1 << 31)) return fail(TM_ERR_TOO_LARGE, "too many blocks");
-        const size_t smem = (size_t)p.L0 * kCols * 3 + (size_t)kSegs * kCols * 4;
-        if (smem > 48 * 1024) {
-            TM_CHECK_CUDA(cudaFuncSetAttribute(edt_c0_smem_kernel<float>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            TM_CHECK_CUDA(cudaFuncSetAttribute(edt_c0_smem_kernel<uint8_t>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        }
-        // after the shell search: overlap this launch with its last CTAs, one
-        // resident wave striding over the column blocks
-        if (in_dtype == TM_F32) {
-            const float *in = static_cast<const float *>(input);
-            if (todo) {
-                const int64_t grid = std::min<int64_t>(blocks, wave_ctas(edt_c0_smem_kernel<float>, kCols * kSegs, smem));
-                TM_CHECK_CUDA(launch_pdl(edt_c0_smem_kernel<float>, dim3((unsigned)grid), dim3(kCols * kSegs), smem,
-                                         stream, in, c1, p, (const int *)todo));
-            } else {
-                edt_c0_smem_kernel<float><<<(unsigned)blocks, kCols * kSegs, smem, stream>>>(in, c1, p, todo);
-            }
-        } else {
-            const uint8_t *in = static_cast<const uint8_t *>(input);
-            if (todo) {
-                const int64_t grid =
-                    std::min<int64_t>(blocks, wave_ctas(edt_c0_smem_kernel<uint8_t>, kCols * kSegs, smem));
-                TM_CHECK_CUDA(launch_pdl(edt_c0_smem_kernel<uint8_t>, dim3((unsigned)grid), dim3(kCols * kSegs),
-                                         smem, stream, in, c1, p, (const int *)todo));
-            } else {
-                edt_c0_smem_kernel<uint8_t><<<(unsigned)blocks, kCols * kSegs, smem, stream>>>(in, c1, p, todo);
-            }
-        }
-        TM_LAUNCH_CHECK("edt_c0_smem_kernel");
-    } else {
-        const int64_t nlines0 = g.batch * inner0;
-        const unsigned b0 = (unsigned)ceil_div(nlines0, 128);
-        if (in_dtype == TM_F32)
-            edt_c0_kernel<float><<<b0, 128, 0, stream>>>(static_cast<const float *>(input), c1, p);
-        else
-            edt_c0_kernel<uint8_t><<<b0, 128, 0, stream>>>(static_cast<const uint8_t *>(input), c1, p);
-        TM_LAUNCH_CHECK("edt_c0_kernel");
-    }
-    // passes 1 + 2 fused per plane when the plane fits on chip
-    if (fused) {
-        const size_t smem = c12_smem(p.L1, p.L2).total;
-        const int64_t blocks = g.batch * (int64_t)p.L0;
-        if (blocks >= ((int64_t)1 << 31)) return fail(TM_ERR_TOO_LARGE, "too many blocks");
-        if (smem > 48 * 1024)
-            TM_CHECK_CUDA(cudaFuncSetAttribute(edt_c12_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem));
-        // launched after pass 0 (whose kernel runs normally when there is no shell search)
-        const int64_t grid = todo ? std::min<int64_t>(blocks, wave_ctas(edt_c12_kernel, kC12Threads, smem)) : blocks;
-        TM_CHECK_CUDA(launch_pdl(edt_c12_kernel, dim3((unsigned)grid), dim3(kC12Threads), smem, stream,
-                                 (const int16_t *)c1, dist, indices, sqdist, p, (const int *)todo));
-        TM_LAUNCH_CHECK("edt_c12_kernel");
-        return TM_OK;
-    }
-    // pass 1 (3-D)
-    if (g.ndim == 3) {
-        const int64_t blocks = g.batch * (int64_t)p.L0 * ceil_div(p.L2, kCols);
-        if (blocks >= ((int64_t)1 << 31)) return fail(TM_ERR_TOO_LARGE, "too many blocks");
-        const size_t smem = (size_t)(p.L1 + kPadTop + kPadBot) * kCols * 6 + kCols * sizeof(int);
-        if (smem > 48 * 1024)
-            TM_CHECK_CUDA(cudaFuncSetAttribute(edt_c1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        edt_c1_kernel<<<(unsigned)blocks, kCols * kSegs, smem, stream>>>(c1, c2, stack1, p);
-        TM_LAUNCH_CHECK("edt_c1_kernel");
-    }
-    // pass 2
-    const int L = g.ndim == 3 ? p.L2 : p.L1;
-    const size_t per_warp = (size_t)(L + 8) * 8 + (size_t)L * 2;
-    // 16-byte vector path: whole 128-voxel chunks and 16-byte aligned planes
-    auto a16 = [](const void *ptr) { return ((uintptr_t)ptr & 15) == 0; };
-    const bool vec = (L % 128) == 0 && (g.numel % 4) == 0 && a16(dist) && a16(indices) && a16(sqdist);
-    int warps = kC2Warps;
-    while (warps > 1 && per_warp * warps > 160 * 1024) warps >>= 1;
-    const int64_t nlines2 = g.numel / L;
-    const unsigned b2 = (unsigned)ceil_div(nlines2, warps);
-    const size_t smem2 = per_warp * warps + kSqrtTab * sizeof(float);
-    auto launch2 = [&](auto kernel, const void *cin) -> int {
-        if (smem2 > 48 * 1024)
-            TM_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
-        kernel<<<b2, warps * 32, smem2, stream>>>(cin, dist, indices, sqdist, p, warps);
-        return TM_OK;
-    };
-    int st;
-    if (g.ndim == 3)
-        st = vec ? launch2(edt_c2_kernel<true, true>, c2) : launch2(edt_c2_kernel<true, false>, c2);
-    else
-        st = vec ? launch2(edt_c2_kernel<false, true>, c1) : launch2(edt_c2_kernel<false, false>, c1);
+    int st = in_dtype == TM_F32 ? launch_bits0(static_cast<const float *>(input), c1, p, todo, stream)
+                                : launch_bits0(static_cast<const uint8_t *>(input), c1, p, todo, stream);
     if (st != TM_OK) return st;
-    TM_LAUNCH_CHECK("edt_c2_kernel");
-    return TM_OK;
+    // lines per tile: 8 long rows, 32 short ones or columns; 512 threads where the staged
+    // lines (68 KB at 1333 voxels) leave room for few CTAs
+    auto rows = [&](auto mode, auto out, const void *src, int L) -> int {
+        constexpr int M = decltype(mode)::value, O = decltype(out)::value;
+        if (L <= kShortLine) return launch_lines<M, 32, 256, O>(src, nullptr, dist, indices, sqdist, p, todo, stream);
+        if (L <= kMediumLine) return launch_lines<M, 8, 256, O>(src, nullptr, dist, indices, sqdist, p, todo, stream);
+        return launch_lines<M, 8, 512, O>(src, nullptr, dist, indices, sqdist, p, todo, stream);
+    };
+    const std::integral_constant<int, 0> k0;
+    const std::integral_constant<int, 1> k1;
+    const std::integral_constant<int, 2> k2;
+    const bool all = indices || sqdist;
+    if (g.ndim == 2) return all ? rows(k0, k1, c1, p.L1) : rows(k0, k0, c1, p.L1);
+    st = p.L2 <= 16 ? launch_lines<1, 8, 256, 0>(c1, c2, nullptr, nullptr, nullptr, p, todo, stream)
+                    : launch_lines<1, 32, 256, 0>(c1, c2, nullptr, nullptr, nullptr, p, todo, stream);
+    if (st != TM_OK) return st;
+    return all ? rows(k2, k1, c2, p.L2) : rows(k2, k0, c2, p.L2);
 }
 
 

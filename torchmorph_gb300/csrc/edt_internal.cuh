@@ -24,10 +24,18 @@ int ragged_edt3_run(const void *input, int in_f32, const ReItem *items, int nite
                     int max_line, int16_t *c1, float *dist, int32_t *indices, int32_t *sqdist, GridControl *ctl,
                     cudaStream_t stream);
 
-bool edt_compact_eligible(const Geometry &g, bool unit);
+// Spacing of an item on the integer passes: squared voxel sizes in units of unit2.
+struct EdtSpacing {
+    uint32_t w[3];
+    float unit2;
+    bool scaled;  // some axis is not 1
+};
+
+// Whether the fast path takes the shape and spacing (sampling NULL: unit); fills *spacing.
+bool edt_compact_eligible(const Geometry &g, const float *sampling, EdtSpacing *spacing);
 size_t edt_compact_workspace(const Geometry &g);
-int edt_compact_run(const void *input, int in_dtype, const Geometry &g, float *dist, int32_t *indices,
-                    int32_t *sqdist, unsigned char *ws, cudaStream_t stream);
+int edt_compact_run(const void *input, int in_dtype, const Geometry &g, const EdtSpacing &spacing, float *dist,
+                    int32_t *indices, int32_t *sqdist, unsigned char *ws, cudaStream_t stream);
 
 // Chamfer distances without indices for 3-D items (bitmap shell search);
 // items it cannot finish are marked in *todo_out (device int per item) for

@@ -58,7 +58,8 @@ extern "C" int tm_edt_noalloc(const void *input, int in_dtype, int64_t batch, in
     if (!input) return fail(TM_ERR_INVALID_ARGUMENT, "input is NULL");
     if (in_dtype != TM_F32 && in_dtype != TM_U8) return fail(TM_ERR_INVALID_ARGUMENT, "unknown input dtype %d", in_dtype);
     if (!dist && !indices && !sqdist) return fail(TM_ERR_INVALID_ARGUMENT, "at least one output must be requested");
-    if (!edt_compact_eligible(g, true))
+    EdtSpacing spacing;
+    if (!edt_compact_eligible(g, nullptr, &spacing) || (g.ndim == 3 && g.shape[1] > 256))
         return fail(TM_ERR_UNSUPPORTED,
                     "tm_edt_noalloc handles 2-D or 3-D items with unit spacing only (use tm_edt with a workspace)");
     const size_t need = edt_compact_workspace(g);
@@ -70,5 +71,5 @@ extern "C" int tm_edt_noalloc(const void *input, int in_dtype, int64_t batch, in
     unsigned char *scratch = nullptr;
     st = scratch_for_current_device(&scratch);
     if (st != TM_OK) return st;
-    return edt_compact_run(input, in_dtype, g, dist, indices, sqdist, scratch, (cudaStream_t)stream);
+    return edt_compact_run(input, in_dtype, g, spacing, dist, indices, sqdist, scratch, (cudaStream_t)stream);
 }
