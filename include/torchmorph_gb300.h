@@ -205,13 +205,16 @@ int tm_binary_dilation(const uint8_t *in, uint8_t *out, int64_t batch, int ndim,
                        const int64_t *shape, const uint8_t *structure, const int64_t *sshape,
                        const int64_t *origin, int border_value, tm_stream_t stream);
 
-/* One-pass binary opening / closing (one iteration, no mask) of 1-D or 2-D
- * items on bit-packed tiles: the first operator over the tile grown by the
+/* One-pass binary opening / closing (one iteration, no mask) of 1-D, 2-D or
+ * 3-D items on bit-packed tiles: the first operator over the tile grown by the
  * second's halo stays on chip, positions outside the item read border_value
  * in both operators -- equal to the reference's two calls
  * (torchmorph/morphology/binary.py:231-290).  Arguments as for
  * tm_binary_erosion; TM_ERR_UNSUPPORTED when a structure offset reaches
- * beyond 16 rows or 32 columns, where the caller composes the operators.
+ * beyond 16 rows or 32 columns (3-D items: 2 planes, 2 rows or 16 columns, or
+ * a structure of more than 128 voxels), where the caller composes the
+ * operators.  tm_binary_erosion / tm_binary_dilation of 3-D items run on the
+ * same tiles within these limits.
  * 1-D / 2-D tm_binary_erosion / tm_binary_dilation with elements other than
  * full boxes run on the same bit tiles. */
 int tm_binary_opening(const uint8_t *in, uint8_t *out, int64_t batch, int ndim, const int64_t *shape,

@@ -192,11 +192,11 @@ def _binary(fn_name, input, structure, origin, border_value, out=None):
 
 
 def binary_composite(kind, input, structure, origin, border_value):
-    """One-pass binary opening / closing (one iteration) of 1-D / 2-D items on bit-packed
+    """One-pass binary opening / closing (one iteration) of 1-D to 3-D items on bit-packed
     tiles (tm_binary_opening / tm_binary_closing); None when the structure is beyond the
     kernel's limits, so that the caller composes the operators."""
     name = {"opening": "tm_binary_opening", "closing": "tm_binary_closing"}[kind]
-    if structure.dim() > 2:
+    if structure.dim() > 3:
         return None
     out = torch.empty_like(input)
     try:

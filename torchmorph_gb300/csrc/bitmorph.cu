@@ -624,18 +624,23 @@ int uniform_open(int kind, const uint8_t *in, uint8_t *out, int64_t batch, int n
                  const uint8_t *structure, const int64_t *sshape, const int64_t *origin, int border_value,
                  tm_stream_t stream) {
     using namespace tmc;
-    if (ndim != 1 && ndim != 2) return fail(TM_ERR_UNSUPPORTED, "fused binary opening / closing: 1-D or 2-D items");
+    if (ndim < 1 || ndim > 3) return fail(TM_ERR_UNSUPPORTED, "fused binary opening / closing: 1-D to 3-D items");
     if (batch < 1 || !shape) return fail(TM_ERR_INVALID_ARGUMENT, "empty batch or NULL shape");
     for (int d = 0; d < ndim; d++)
         if (shape[d] < 1) return fail(TM_ERR_INVALID_ARGUMENT, "empty item");
     int st = check_binary_args(in, out, structure, sshape, origin, ndim);
     if (st != TM_OK) return st;
     bool done = false;
-    st = bitmorph_uniform(kind, in, out, batch, ndim, shape, structure, sshape, origin, border_value,
-                          (cudaStream_t)stream, &done);
+    if (ndim == 3)
+        st = bitmorph3d_uniform(kind, in, out, batch, shape, structure, sshape, origin, border_value,
+                                (cudaStream_t)stream, &done);
+    else
+        st = bitmorph_uniform(kind, in, out, batch, ndim, shape, structure, sshape, origin, border_value,
+                              (cudaStream_t)stream, &done);
     if (st != TM_OK) return st;
     if (!done)
-        return fail(TM_ERR_UNSUPPORTED, "structure beyond the fused kernel (taps within 16 rows / 32 columns)");
+        return fail(TM_ERR_UNSUPPORTED, "structure beyond the fused kernel (taps within 16 rows / 32 columns; 3-D: 2 "
+                                        "planes, 2 rows, 16 columns)");
     return TM_OK;
 }
 

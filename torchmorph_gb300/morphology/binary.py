@@ -156,13 +156,13 @@ def binary_hit_or_miss(input, structure1=None, structure2=None, output=None, ori
 
 
 def _one_pass(kind, input, structure, iterations, mask, output, border_value, origin):
-    """The one-pass opening / closing of 1-D / 2-D items (one iteration, no mask) on
+    """The one-pass opening / closing of 1-D to 3-D items (one iteration, no mask) on
     bit-packed tiles; None where the reference's composition of two operators runs."""
     if iterations != 1 or mask is not None:
         return None
     nd = validate_bcs_input(input)
     validate_output(input, output)
-    if nd > 2:
+    if nd > 3:
         return None
     if structure is None:
         structure = _default_structure(nd)
@@ -183,7 +183,7 @@ def _one_pass(kind, input, structure, iterations, mask, output, border_value, or
 
 def binary_opening(input, structure=None, iterations=1, mask=None, output=None, border_value=False,
                    origin=0) -> Tensor:
-    """Erosion followed by dilation (1-D / 2-D, one iteration: one pass)."""
+    """Erosion followed by dilation (1-D to 3-D, one iteration: one pass)."""
     res = _one_pass("opening", input, structure, iterations, mask, output, border_value, origin)
     if res is not None:
         return res
@@ -193,7 +193,7 @@ def binary_opening(input, structure=None, iterations=1, mask=None, output=None, 
 
 def binary_closing(input, structure=None, iterations=1, mask=None, output=None, border_value=False,
                    origin=0) -> Tensor:
-    """Dilation followed by erosion (1-D / 2-D, one iteration: one pass)."""
+    """Dilation followed by erosion (1-D to 3-D, one iteration: one pass)."""
     res = _one_pass("closing", input, structure, iterations, mask, output, border_value, origin)
     if res is not None:
         return res
