@@ -138,6 +138,45 @@ __device__ __forceinline__ void window_run(const T *src, int step, int k, T *res
     }
 }
 
+// kRun outputs as above from the fewest shared-memory reads: a van Herk/Gil-Werman split
+// of RUN outputs reads every element of its span once (k + RUN - 1 reads, about 2 k + 2
+// RUN combines), so windows of 4 .. 7 take two runs of 4.  Windows below 4 are read tap by tap.
+template <typename T, bool MAX, int RUN>
+__device__ __forceinline__ void van_herk_run(const T *src, int step, int k, T *res) {
+    using Op = MorphOp<T, MAX>;
+    T mid = src[(RUN - 1) * step];
+    for (int t = RUN; t < k; t++) mid = Op::combine(mid, src[t * step]);
+    T suf[RUN];
+    suf[RUN - 1] = mid;
+#pragma unroll
+    for (int j = RUN - 2; j >= 0; j--) suf[j] = Op::combine(src[j * step], suf[j + 1]);
+    res[0] = suf[0];
+    T pre = src[k * step];
+#pragma unroll
+    for (int j = 1; j < RUN; j++) {
+        res[j] = Op::combine(suf[j], pre);
+        if (j + 1 < RUN) pre = Op::combine(pre, src[(k + j) * step]);
+    }
+}
+
+template <typename T, bool MAX>
+__device__ __forceinline__ void window_run_split(const T *src, int step, int k, T *res) {
+    using Op = MorphOp<T, MAX>;
+    if (k >= kRun) {
+        van_herk_run<T, MAX, kRun>(src, step, k, res);
+    } else if (k >= kRun / 2) {
+        van_herk_run<T, MAX, kRun / 2>(src, step, k, res);
+        van_herk_run<T, MAX, kRun / 2>(src + (kRun / 2) * step, step, k, res + kRun / 2);
+    } else {
+#pragma unroll
+        for (int j = 0; j < kRun; j++) {
+            T acc = src[j * step];
+            for (int t = 1; t < k; t++) acc = Op::combine(acc, src[(j + t) * step]);
+            res[j] = acc;
+        }
+    }
+}
+
 // Row pass then column pass of one staged tile: `tile` points at the first
 // input column the tile needs (row stride ld), `rows` receives the row-pass
 // result (RH x kTileW at pitch kRowsPitch); outputs go to dst at (y0.., x0..).
