@@ -95,6 +95,43 @@ constexpr int kRowsPitch = kTileW + 1;
 // banks (the row pass gives consecutive rows to consecutive threads).
 __host__ __device__ inline int stage_pitch(int kw) { return (kTileW + kw - 1 + (kRun - 1)) | 1; }
 
+// Stage rows [gy0, gy0 + RH) x columns [gx0, gx0 + RW) of one H x W image into shared
+// memory (row stride ld), mapping out-of-image coordinates with the border mode.  Warp w
+// takes rows w, w + 8, ...; a lane maps its up to 5 columns of a chunk once for all rows
+// and issues the loads of 2 rows before it stores any, so border tiles cost what
+// interior ones do and a warp keeps 10 loads in flight.
+template <typename T>
+__device__ __forceinline__ void stage_tile(const T *__restrict__ src, int H, int W, int gy0, int gx0, int RH, int RW,
+                                           int ld, int mode, T cval, T *tile) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int nwarps = kFlatThreads / 32, RB = 2, NC = 5;
+    for (int cb = lane; cb < RW; cb += 32 * NC) {
+        int mx[NC];  // -1: the constant; columns past the region repeat one inside it, unstored
+#pragma unroll
+        for (int j = 0; j < NC; j++) mx[j] = map_coord(gx0 + min(cb + 32 * j, RW - 1), W, mode);
+        const int last = (RW - 1 - cb) / 32;  // chunk columns 0 .. last are inside the region
+        for (int rb = warp; rb < RH; rb += nwarps * RB) {
+            T v[RB][NC];
+#pragma unroll
+            for (int k = 0; k < RB; k++) {
+                const int my = map_coord(gy0 + min(rb + nwarps * k, RH - 1), H, mode);
+                const T *row = src + (int64_t)max(my, 0) * W;
+#pragma unroll
+                for (int j = 0; j < NC; j++) v[k][j] = my >= 0 && mx[j] >= 0 ? row[mx[j]] : cval;
+            }
+#pragma unroll
+            for (int k = 0; k < RB; k++) {
+                const int r = rb + nwarps * k;
+                if (r >= RH) break;
+                T *t = tile + r * ld + cb;
+#pragma unroll
+                for (int j = 0; j < NC; j++)
+                    if (j <= last) t[32 * j] = v[k][j];
+            }
+        }
+    }
+}
+
 struct Flat2DParams {
     int H, W;        // item size (1-D items use H = 1)
     int kh, kw;      // window
@@ -103,44 +140,15 @@ struct Flat2DParams {
     int64_t batch;
     float cval;
     float sval;  // constant structure value (flat footprint)
+    FastDiv d_rows;  // divides by kTileH + kh - 1
 };
 
 
-// One run of kRun consecutive outputs of a 1-D sliding window of width k
-// over src[0 .. kRun + k - 2] (src elements `step` apart in shared memory).
-template <typename T, bool MAX>
-__device__ __forceinline__ void window_run(const T *src, int step, int k, T *res) {
-    using Op = MorphOp<T, MAX>;
-    if (k <= kRun) {
-#pragma unroll
-        for (int j = 0; j < kRun; j++) {
-            T acc = src[j * step];
-            for (int t = 1; t < k; t++) acc = Op::combine(acc, src[(j + t) * step]);
-            res[j] = acc;
-        }
-        return;
-    }
-    // van Herk/Gil-Werman split: every window of the run contains the
-    // block [kRun-1, k-1]; the left part is a suffix of [j, kRun-2] and the
-    // right part a prefix of [k, j+k-1].
-    T mid = src[(kRun - 1) * step];
-    for (int t = kRun; t < k; t++) mid = Op::combine(mid, src[t * step]);
-    T suf[kRun];
-    suf[kRun - 1] = mid;
-#pragma unroll
-    for (int j = kRun - 2; j >= 0; j--) suf[j] = Op::combine(src[j * step], suf[j + 1]);
-    T pre = src[k * step];
-    res[0] = suf[0];
-#pragma unroll
-    for (int j = 1; j < kRun; j++) {
-        res[j] = Op::combine(suf[j], pre);
-        if (j + 1 < kRun) pre = Op::combine(pre, src[(k + j) * step]);
-    }
-}
-
-// kRun outputs as above from the fewest shared-memory reads: a van Herk/Gil-Werman split
-// of RUN outputs reads every element of its span once (k + RUN - 1 reads, about 2 k + 2
-// RUN combines), so windows of 4 .. 7 take two runs of 4.  Windows below 4 are read tap by tap.
+// One run of RUN consecutive outputs of a 1-D sliding window of width k >= RUN over
+// src[0 .. RUN + k - 2] (src elements `step` apart in shared memory), by the van Herk/
+// Gil-Werman split: every window of the run contains the block [RUN - 1, k - 1]; the left
+// part is a suffix of [j, RUN - 2], the right part a prefix of [k, j + k - 1].  Every
+// element of the span is read once (k + RUN - 1 reads, about k + 3 RUN combines).
 template <typename T, bool MAX, int RUN>
 __device__ __forceinline__ void van_herk_run(const T *src, int step, int k, T *res) {
     using Op = MorphOp<T, MAX>;
@@ -159,8 +167,10 @@ __device__ __forceinline__ void van_herk_run(const T *src, int step, int k, T *r
     }
 }
 
+// kRun outputs from the fewest reads: one run of 8, two of 4 for windows of 4 .. 7, tap
+// by tap below.
 template <typename T, bool MAX>
-__device__ __forceinline__ void window_run_split(const T *src, int step, int k, T *res) {
+__device__ __forceinline__ void window_run(const T *src, int step, int k, T *res) {
     using Op = MorphOp<T, MAX>;
     if (k >= kRun) {
         van_herk_run<T, MAX, kRun>(src, step, k, res);
@@ -178,53 +188,40 @@ __device__ __forceinline__ void window_run_split(const T *src, int step, int k, 
 }
 
 // Row pass then column pass of one staged tile: `tile` points at the first
-// input column the tile needs (row stride ld), `rows` receives the row-pass
+// input column the tile needs (odd row stride ld), `rows` receives the row-pass
 // result (RH x kTileW at pitch kRowsPitch); outputs go to dst at (y0.., x0..).
+// (RH rows of the region and the columns inside the item are computed; d_rows divides by RH.)
 template <typename T, bool MAX>
 __device__ __forceinline__ void flat_tile_compute(const T *tile, int ld, T *rows, const Flat2DParams &p, T *dst,
                                                   int x0, int y0) {
-    using Op = MorphOp<T, MAX>;
     const int RH = kTileH + p.kh - 1;
-    if (p.kw <= kRun) {
-        // narrow windows: one output per thread, adjacent lanes on adjacent
-        // columns, so every shared-memory access of a warp is conflict free
-        for (int w = threadIdx.x; w < RH * kTileW; w += kFlatThreads) {
-            const int r = w / kTileW, c = w % kTileW;
-            const T *src = tile + r * ld + c;
-            T acc = src[0];
-            for (int t = 1; t < p.kw; t++) acc = Op::combine(acc, src[t]);
-            rows[r * kRowsPitch + c] = acc;
-        }
-    } else {
-        const int runs_per_row = kTileW / kRun;
-        // an odd row stride: consecutive threads take the same run of consecutive
-        // rows (conflict-free); otherwise consecutive runs of one row
-        const bool by_rows = (ld & 1) != 0;
-        for (int w = threadIdx.x; w < RH * runs_per_row; w += kFlatThreads) {
-            const int r = by_rows ? w % RH : w / runs_per_row;
-            const int c = (by_rows ? w / RH : w % runs_per_row) * kRun;
-            T res[kRun];
-            window_run<T, MAX>(tile + r * ld + c, 1, p.kw, res);
+    const int cols = min(kTileW, p.W - x0), outs = min(kTileH, p.H - y0);
+    const int runs = (cols + kRun - 1) / kRun;
+    // (every row of the region, also below the outputs of a tile at the item's end: the
+    // work unit's division stays a constant one; those rows are stale and unused)
+    for (int w = threadIdx.x; w < RH * runs; w += kFlatThreads) {
+        // consecutive threads take the same run of consecutive rows (odd row stride)
+        const int u = (int)fdiv(w, p.d_rows), r = w - u * RH;
+        if (r >= outs + p.kh - 1) continue;
+        const int c = kRun * u;
+        T res[kRun];
+        window_run<T, MAX>(tile + r * ld + c, 1, p.kw, res);
 #pragma unroll
-            for (int j = 0; j < kRun; j++) rows[r * kRowsPitch + c + j] = res[j];
-        }
+        for (int j = 0; j < kRun; j++) rows[r * kRowsPitch + c + j] = res[j];
     }
     __syncthreads();
     const int runs_per_col = kTileH / kRun;
     for (int w = threadIdx.x; w < kTileW * runs_per_col; w += kFlatThreads) {
-        int c = w % kTileW, r = (w / kTileW) * kRun;
-        int gx = x0 + c;
+        const int c = w % kTileW, r = (w / kTileW) * kRun;
+        if (c >= cols || r >= outs) continue;
         // kTileH is a multiple of kRun, so the run reads rows
         // r .. r + kRun + kh - 2 <= RH - 1: always inside the row buffer
         T res[kRun];
         window_run<T, MAX>(rows + r * kRowsPitch + c, kRowsPitch, p.kh, res);
-        if (gx < p.W) {
+        T *o = dst + (int64_t)(y0 + r) * p.W + x0 + c;
 #pragma unroll
-            for (int j = 0; j < kRun; j++) {
-                int gy = y0 + r + j;
-                if (gy < p.H) __stcs(dst + (int64_t)gy * p.W + gx, MorphOp<T, MAX>::apply(res[j], p.sval));
-            }
-        }
+        for (int j = 0; j < kRun; j++, o += p.W)
+            if (r + j < outs) __stcs(o, MorphOp<T, MAX>::apply(res[j], p.sval));
     }
 }
 

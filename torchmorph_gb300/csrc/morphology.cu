@@ -38,42 +38,20 @@ using namespace morph;
 template <typename T, bool MAX, int KH, int KW>
 __global__ void __launch_bounds__(kFlatThreads) flat2d_kernel(const T *__restrict__ in, T *__restrict__ out,
                                                               Flat2DParams p) {
-    using Op = MorphOp<T, MAX>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int RH = kTileH + p.kh - 1;      // loaded rows
     const int RW = kTileW + p.kw - 1;      // loaded columns
     const int RWp = stage_pitch(p.kw);     // padded so full runs never read past a row; odd
     T *tile = reinterpret_cast<T *>(smem_raw);
     T *rows = tile + RH * RWp;             // row-pass result, RH x kTileW at pitch kRowsPitch
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nwarps = kFlatThreads / 32;
-    const T cval = (T)p.cval;
-
     const int x0 = blockIdx.x * kTileW;
     const int y0 = blockIdx.y * kTileH;
     for (int64_t item = blockIdx.z; item < p.batch; item += gridDim.z) {
-        const T *src = in + item * (int64_t)p.H * p.W;
-        T *dst = out + item * (int64_t)p.H * p.W;
-        const int gy0 = y0 + p.lo_y, gx0 = x0 + p.lo_x;
-        const bool interior = gy0 >= 0 && gx0 >= 0 && gy0 + RH <= p.H && gx0 + RW <= p.W;
-        // 1. stage the input tile (coalesced along x), mapping borders
-        for (int r = warp; r < RH; r += nwarps) {
-            int gy = gy0 + r;
-            int my = interior ? gy : map_coord(gy, p.H, p.mode);
-            for (int c = lane; c < RW; c += 32) {
-                int gx = gx0 + c;
-                T v;
-                if (interior) {
-                    v = src[(int64_t)gy * p.W + gx];
-                } else {
-                    int mx = map_coord(gx, p.W, p.mode);
-                    v = (my < 0 || mx < 0) ? cval : src[(int64_t)my * p.W + mx];
-                }
-                tile[r * RWp + c] = v;
-            }
-        }
+        const int64_t off = item * (int64_t)p.H * p.W;
+        stage_tile<T>(in + off, p.H, p.W, y0 + p.lo_y, x0 + p.lo_x, min(RH, p.H - y0 + p.kh - 1),
+                      min(RW, p.W - x0 + p.kw - 1), RWp, p.mode, (T)p.cval, tile);
         __syncthreads();
-        tile_compute<T, MAX, KH, KW>(tile, RWp, rows, p, dst, x0, y0);
+        tile_compute<T, MAX, KH, KW>(tile, RWp, rows, p, out + off, x0, y0);
         __syncthreads();
     }
 }
@@ -150,9 +128,7 @@ __global__ void __launch_bounds__(kFlatThreads) flat2d_tma_kernel(const __grid_c
     const int RW = kTileW + p.kw - 1;
     const size_t buf_bytes = round_up((size_t)RH * tp.bw * sizeof(T), 1024);
     T *buf[2] = {reinterpret_cast<T *>(smem_raw), reinterpret_cast<T *>(smem_raw + buf_bytes)};
-    T *rows = reinterpret_cast<T *>(smem_raw + 2 * buf_bytes);
-    const size_t rows_bytes = KH == 0 ? round_up((size_t)RH * kRowsPitch * sizeof(T), 16) : 0;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw + 2 * buf_bytes + rows_bytes);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw + 2 * buf_bytes);
     if (threadIdx.x == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
@@ -220,8 +196,8 @@ __global__ void __launch_bounds__(kFlatThreads) flat2d_tma_kernel(const __grid_c
             }
             __syncthreads();
         }
-        tile_compute<T, MAX, KH, KW>(buf[s] + off, tp.bw, rows, p, out + item * (int64_t)p.H * p.W, tx * kTileW,
-                                     ty * kTileH);
+        flat_tile_walk<T, MAX, KH, KW>(buf[s] + off, tp.bw, p, out + item * (int64_t)p.H * p.W, tx * kTileW,
+                                       ty * kTileH);
         __syncthreads();
     }
 }
@@ -307,19 +283,13 @@ struct Tap {
     float val;
 };
 
-// Flat 1-D/2-D box: the mapped-border kernel for every tile (or only the
-// border ring when the TMA kernel takes the interior), then the TMA kernel.
+// Compile-time windows: persistent TMA-staged tiles once a batch has a few per SM and its
+// rows are 16-byte aligned (off-centre 3 x 3 on 8 x 4096^2: 205 us, 307 us with a CTA per
+// tile), else a CTA per tile.
 template <typename T, bool MAX, int KH, int KW>
-int launch_flat2d(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, cudaStream_t stream) {
-    const int RH = kTileH + p.kh - 1, RWp = stage_pitch(p.kw);
-    const size_t rows_bytes = KH == 0 ? (size_t)RH * kRowsPitch * sizeof(T) : 0;
-    const size_t smem = (size_t)RH * RWp * sizeof(T) + rows_bytes;
-    if (smem > 48 * 1024)
-        TM_CHECK_CUDA(cudaFuncSetAttribute(flat2d_kernel<T, MAX, KH, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
-    dim3 grid((unsigned)ceil_div(p.W, kTileW), (unsigned)ceil_div(p.H, kTileH),
-              (unsigned)(batch < 65535 ? batch : 65535));
-    // TMA path for the interior tiles: needs 16-byte aligned rows and a box of at most 256 x 256
+int launch_flat2d_small(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, dim3 grid, size_t smem,
+                        cudaStream_t stream) {
+    const int RH = kTileH + p.kh - 1;
     TmaTileParams tp;
     tp.align = 16 / (int)sizeof(T);
     tp.bw = (int)round_up((size_t)(kTileW + p.kw - 1 + tp.align - 1), (size_t)tp.align);
@@ -364,8 +334,7 @@ int launch_flat2d(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, c
     int *status = nullptr;
     st = device_status_word(&status);
     if (st != TM_OK) return st;
-    const size_t tsmem = 2 * round_up((size_t)RH * tp.bw * sizeof(T), 1024) +
-                         (KH == 0 ? round_up((size_t)RH * kRowsPitch * sizeof(T), 16) : 0) + 2 * sizeof(uint64_t) + 1024;
+    const size_t tsmem = 2 * round_up((size_t)RH * tp.bw * sizeof(T), 1024) + 2 * sizeof(uint64_t) + 1024;
     if (tsmem > 220 * 1024) return fail(TM_ERR_UNSUPPORTED, "TMA tile does not fit in shared memory");
     // attribute + occupancy depend only on the instantiation and the smem size: cache the last answer
     static thread_local size_t cached_smem = 0;
@@ -387,6 +356,28 @@ int launch_flat2d(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, c
     flat2d_tma_kernel<T, MAX, KH, KW><<<(unsigned)ctas, kFlatThreads, tsmem, stream>>>(map, in, out, p, tp, status);
     TM_LAUNCH_CHECK("flat2d_tma_kernel");
     return TM_OK;
+}
+
+// Flat 1-D/2-D box, a CTA per tile or persistent TMA-staged tiles.
+template <typename T, bool MAX, int KH, int KW>
+int launch_flat2d(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, cudaStream_t stream) {
+    const int RH = kTileH + p.kh - 1, RWp = stage_pitch(p.kw);
+    const size_t rows_bytes = KH == 0 ? (size_t)RH * kRowsPitch * sizeof(T) : 0;
+    const size_t smem = (size_t)RH * RWp * sizeof(T) + rows_bytes;
+    if (smem > 48 * 1024)
+        TM_CHECK_CUDA(cudaFuncSetAttribute(flat2d_kernel<T, MAX, KH, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem));
+    dim3 grid((unsigned)ceil_div(p.W, kTileW), (unsigned)ceil_div(p.H, kTileH),
+              (unsigned)(batch < 65535 ? batch : 65535));
+    // windows of a runtime size: their row pass wants an odd row pitch, which a TMA box
+    // cannot have (15 x 15 on 4 x 2048^2: 53 us, 98 us through TMA-staged tiles)
+    if constexpr (KH == 0) {
+        flat2d_kernel<T, MAX, KH, KW><<<grid, kFlatThreads, smem, stream>>>(in, out, p);
+        TM_LAUNCH_CHECK("flat2d_kernel");
+        return TM_OK;
+    } else {
+        return launch_flat2d_small<T, MAX, KH, KW>(in, out, p, batch, sms, grid, smem, stream);
+    }
 }
 
 template <typename T, bool MAX>
@@ -472,6 +463,7 @@ int run_morphology(const T *in, T *out, int64_t batch, int ndim, const int64_t *
         p.batch = batch;
         p.cval = cval;
         p.sval = first_val;
+        p.d_rows = make_fastdiv(kTileH + p.kh - 1);
         if (p.kh > 4096 || p.kw > 4096) goto stencil;  // tile would not fit on chip
         {
             const int RH = kTileH + p.kh - 1, RW = stage_pitch(p.kw);
@@ -488,9 +480,11 @@ int run_morphology(const T *in, T *out, int64_t batch, int ndim, const int64_t *
                     if (st != TM_OK || done) return st;
                 }
             }
-            if (p.kh == 3 && p.kw == 3) return launch_flat2d<T, MAX, 3, 3>(in, out, p, batch, sms, stream);
-            if (p.kh == 5 && p.kw == 5) return launch_flat2d<T, MAX, 5, 5>(in, out, p, batch, sms, stream);
-            if (p.kh == 1 && p.kw == 3) return launch_flat2d<T, MAX, 1, 3>(in, out, p, batch, sms, stream);
+            if constexpr (sizeof(T) == 4) {  // (binary windows of this size run on bit tiles)
+                if (p.kh == 3 && p.kw == 3) return launch_flat2d<T, MAX, 3, 3>(in, out, p, batch, sms, stream);
+                if (p.kh == 5 && p.kw == 5) return launch_flat2d<T, MAX, 5, 5>(in, out, p, batch, sms, stream);
+                if (p.kh == 1 && p.kw == 3) return launch_flat2d<T, MAX, 1, 3>(in, out, p, batch, sms, stream);
+            }
             return launch_flat2d<T, MAX, 0, 0>(in, out, p, batch, sms, stream);
         }
     }

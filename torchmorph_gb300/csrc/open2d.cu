@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kOThreads, 2) open2d_kernel(const float *__res
     for (int w = threadIdx.x; w < RH0 * runs_w1; w += kOThreads) {
         const int u = fdiv(w, p.d_rows0), r = w - u * RH0, c = start(u, RW1);
         float res[kRun];
-        window_run_split<float, MAX1>(s0 + r * P0 + c, 1, p.kw, res);
+        window_run<float, MAX1>(s0 + r * P0 + c, 1, p.kw, res);
 #pragma unroll
         for (int j = 0; j < kRun; j++) rowb[r * P1 + c + j] = res[j];
     }
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kOThreads, 2) open2d_kernel(const float *__res
     for (int w = threadIdx.x; w < RW1 * runs_h1; w += kOThreads) {
         const int u = fdiv(w, p.d_cols1), c = w - u * RW1, r = start(u, RH1);
         float res[kRun];
-        window_run_split<float, MAX1>(rowb + r * P1 + c, P1, p.kh, res);
+        window_run<float, MAX1>(rowb + r * P1 + c, P1, p.kh, res);
 #pragma unroll
         for (int j = 0; j < kRun; j++) s0[(r + j) * P0 + c] = Op1::apply(res[j], p.sval);
     }
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kOThreads, 2) open2d_kernel(const float *__res
     for (int w = threadIdx.x; w < RH1 * (kOTileW / kRun); w += kOThreads) {
         const int u = fdiv(w, p.d_rows1), r = w - u * RH1, c = kRun * u;
         float res[kRun];
-        window_run_split<float, !MAX1>(s0 + r * P0 + c, 1, p.kw, res);
+        window_run<float, !MAX1>(s0 + r * P0 + c, 1, p.kw, res);
 #pragma unroll
         for (int j = 0; j < kRun; j++) rowb[r * P1 + c + j] = res[j];
     }
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kOThreads, 2) open2d_kernel(const float *__res
 #pragma unroll
             for (int j = 0; j < kRun; j++) x[j] = yy + j < p.H ? __ldg(src + (int64_t)(yy + j) * p.W + xx) : 0.0f;
         }
-        window_run_split<float, !MAX1>(rowb + r * P1 + c, P1, p.kh, res);
+        window_run<float, !MAX1>(rowb + r * P1 + c, P1, p.kh, res);
         const bool column_in = xx >= p.rx0 && xx < p.rx1;
 #pragma unroll
         for (int j = 0; j < kRun; j++) {

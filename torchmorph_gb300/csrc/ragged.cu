@@ -52,6 +52,7 @@ static_assert(sizeof(PlanHeader) == 256, "plan header is 256 bytes");
 struct RaggedWindow {
     int kh, kw, lo_y, lo_x, mode;
     float cval, sval;
+    FastDiv d_rows;
 };
 
 constexpr int kMaxTaps = 256;
@@ -62,60 +63,6 @@ struct RaggedTaps {
     int8_t dy[kMaxTaps], dx[kMaxTaps];
     float val[kMaxTaps];
 };
-
-// Stage rows [gy0, gy0 + RH) x columns [gx0, gx0 + RW) of one image into
-// shared memory (row stride ld), mapping out-of-image coordinates.  Warp w
-// takes rows w, w + 8, ...; a lane issues the loads of 2 rows x up to 5
-// column chunks before it stores any, so a warp keeps many loads in flight
-// (tiles inside the image; border tiles map every coordinate, one row at a
-// time).
-template <typename T>
-__device__ __forceinline__ void stage_tile(const T *src, int H, int W, int gy0, int gx0, int RH, int RW, int ld,
-                                           int mode, T cval, T *tile) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int nwarps = kFlatThreads / 32, RB = 2, NC = 5;
-    const bool interior = gy0 >= 0 && gx0 >= 0 && gy0 + RH <= H && gx0 + RW <= W;
-    if (interior) {
-        for (int rb = warp; rb < RH; rb += nwarps * RB)
-            for (int cb = 0; cb < RW; cb += 32 * NC) {
-                T v[RB][NC];
-#pragma unroll
-                for (int k = 0; k < RB; k++)
-#pragma unroll
-                    for (int j = 0; j < NC; j++) {
-                        const int r = rb + nwarps * k, c = cb + lane + 32 * j;
-                        if (r < RH && c < RW) v[k][j] = src[(int64_t)(gy0 + r) * W + gx0 + c];
-                    }
-#pragma unroll
-                for (int k = 0; k < RB; k++)
-#pragma unroll
-                    for (int j = 0; j < NC; j++) {
-                        const int r = rb + nwarps * k, c = cb + lane + 32 * j;
-                        if (r < RH && c < RW) tile[r * ld + c] = v[k][j];
-                    }
-            }
-        return;
-    }
-    for (int r = warp; r < RH; r += nwarps) {
-        const int my = map_coord(gy0 + r, H, mode);
-        for (int cb = 0; cb < RW; cb += 32 * NC) {
-            T v[NC];
-#pragma unroll
-            for (int j = 0; j < NC; j++) {
-                const int c = cb + lane + 32 * j;
-                if (c < RW) {
-                    const int mx = map_coord(gx0 + c, W, mode);
-                    v[j] = (my < 0 || mx < 0) ? cval : src[(int64_t)my * W + mx];
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < NC; j++) {
-                const int c = cb + lane + 32 * j;
-                if (c < RW) tile[r * ld + c] = v[j];
-            }
-        }
-    }
-}
 
 template <typename T, bool MAX, int KH, int KW>
 __global__ void __launch_bounds__(kFlatThreads) ragged_flat_kernel(const T *__restrict__ in, T *__restrict__ out,
@@ -147,7 +94,10 @@ __global__ void __launch_bounds__(kFlatThreads) ragged_flat_kernel(const T *__re
         p.batch = 1;
         p.cval = w.cval;
         p.sval = w.sval;
-        stage_tile<T>(in + it.off, it.H, it.W, y0 + w.lo_y, x0 + w.lo_x, RH, RW, RWp, w.mode, (T)w.cval, tile);
+        p.d_rows = w.d_rows;
+        // (the rows and columns that outputs inside the image read)
+        stage_tile<T>(in + it.off, it.H, it.W, y0 + w.lo_y, x0 + w.lo_x, min(RH, it.H - y0 + w.kh - 1),
+                      min(RW, it.W - x0 + w.kw - 1), RWp, w.mode, (T)w.cval, tile);
         __syncthreads();
         tile_compute<T, MAX, KH, KW>(tile, RWp, rows, p, out + it.off, x0, y0);
         __syncthreads();
@@ -332,9 +282,12 @@ int run_ragged(const T *in, T *out, const void *plan, size_t plan_bytes, int64_t
         w.mode = mode;
         w.cval = cval;
         w.sval = first;
-        if (kh == 3 && kw == 3) return launch_ragged_flat<T, MAX, 3, 3>(in, out, hdr, items, w, s);
-        if (kh == 5 && kw == 5) return launch_ragged_flat<T, MAX, 5, 5>(in, out, hdr, items, w, s);
-        if (kh == 1 && kw == 3) return launch_ragged_flat<T, MAX, 1, 3>(in, out, hdr, items, w, s);
+        w.d_rows = make_fastdiv(kTileH + kh - 1);
+        if constexpr (sizeof(T) == 4) {  // (binary windows of this size run on bit tiles)
+            if (kh == 3 && kw == 3) return launch_ragged_flat<T, MAX, 3, 3>(in, out, hdr, items, w, s);
+            if (kh == 5 && kw == 5) return launch_ragged_flat<T, MAX, 5, 5>(in, out, hdr, items, w, s);
+            if (kh == 1 && kw == 3) return launch_ragged_flat<T, MAX, 1, 3>(in, out, hdr, items, w, s);
+        }
         return launch_ragged_flat<T, MAX, 0, 0>(in, out, hdr, items, w, s);
     }
     if (n > kMaxTaps) return fail(TM_ERR_UNSUPPORTED, "ragged footprints are limited to %d active taps", kMaxTaps);
