@@ -9,8 +9,6 @@ through PyTorch's caching allocator, as in the reference.
 
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
 from . import _lib
@@ -24,16 +22,13 @@ def _require(cond: bool, msg: str) -> None:
 
 
 def _batch_shape(t: torch.Tensor):
-    _require(t.dim() >= 3, "input must be (B, C, spatial...) with at least 3 dimensions")
-    return t.shape[0] * t.shape[1], list(t.shape[2:])
+    shape = t.shape
+    _require(len(shape) >= 3, "input must be (B, C, spatial...) with at least 3 dimensions")
+    return shape[0] * shape[1], shape[2:]
 
 
-def _host_f32(t: torch.Tensor):
-    return ctypes.cast(t.data_ptr(), _lib.F32P)
-
-
-def _host_u8(t: torch.Tensor):
-    return ctypes.cast(t.data_ptr(), _lib.U8P)
+_host_f32 = _lib.ctypes_f32
+_host_u8 = _lib.ctypes_u8
 
 
 def _workspace(nbytes: int, device) -> torch.Tensor | None:
@@ -64,7 +59,7 @@ def _grey(fn_name, input, structure, footprint, origin, mode, cval):
     batch, shape = _batch_shape(input)
     out = torch.empty_like(input)
     lib = _lib.load()
-    with torch.cuda.device(input.device):
+    with _lib.on_device(input.device):
         st = getattr(lib, fn_name)(
             _lib.ptr(input), _lib.ptr(out), batch, nd, _lib.i64_array(shape), _host_f32(structure),
             _host_u8(footprint) if use_fp else None, _lib.i64_array(structure.shape),
@@ -107,7 +102,7 @@ def grey_composite(kind, input, structure, footprint, origin, mode, cval):
     batch, shape = _batch_shape(input)
     out = torch.empty_like(input)
     lib = _lib.load()
-    with torch.cuda.device(input.device):
+    with _lib.on_device(input.device):
         st = getattr(lib, name)(
             _lib.ptr(input), _lib.ptr(out), batch, nd, _lib.i64_array(shape), _host_f32(structure),
             _host_u8(footprint) if use_fp else None, _lib.i64_array(structure.shape),
@@ -129,7 +124,7 @@ def _grey_arg(fn_name, input, structure, footprint, origin, mode, cval):
     out = torch.empty_like(input)
     arg = torch.empty(input.shape, dtype=torch.uint8, device=input.device)
     lib = _lib.load()
-    with torch.cuda.device(input.device):
+    with _lib.on_device(input.device):
         st = getattr(lib, fn_name)(
             _lib.ptr(input), _lib.ptr(out), _lib.ptr(arg), batch, nd, _lib.i64_array(shape),
             _host_f32(structure), _host_u8(footprint) if use_fp else None,
@@ -157,7 +152,7 @@ def grey_morphology_backward(grad_output, arg, sshape, footprint, origin, mode, 
     use_fp = footprint.numel() != 0
     name = "tm_grey_dilation_backward" if dilation else "tm_grey_erosion_backward"
     lib = _lib.load()
-    with torch.cuda.device(g.device):
+    with _lib.on_device(g.device):
         st = getattr(lib, name)(
             _lib.ptr(g), _lib.ptr(arg), _lib.ptr(gin), batch, nd, _lib.i64_array(shape),
             _host_u8(footprint) if use_fp else None, _lib.i64_array(sshape), _lib.i64_array(origin),
@@ -182,7 +177,7 @@ def _binary(fn_name, input, structure, origin, border_value, out=None):
     if out is None:
         out = torch.empty_like(input)
     lib = _lib.load()
-    with torch.cuda.device(input.device):
+    with _lib.on_device(input.device):
         st = getattr(lib, fn_name)(
             _lib.ptr(input), _lib.ptr(out), batch, nd, _lib.i64_array(shape), _host_u8(structure),
             _lib.i64_array(structure.shape), _lib.i64_array(origin), int(bool(border_value)),
@@ -250,7 +245,7 @@ def edt(input, sampling=None, return_distances=True, return_indices=False, sqdis
             (nd, *input.shape), dtype=torch.int32, device=dev)
     sq = torch.empty(input.shape, dtype=torch.int32, device=dev) if sqdist else None
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         shp = _lib.i64_array(shape)
         samp = None if sampling is None else _lib.f32_array(sampling)
         ws = _workspace(lib.tm_edt_workspace_size(batch, nd, shp, samp), dev)
@@ -287,7 +282,7 @@ def cdt(input, metric="chessboard", return_distances=True, return_indices=False,
         ind = indices_out if indices_out is not None else torch.empty(
             (nd, *input.shape), dtype=torch.int32, device=dev)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         shp = _lib.i64_array(shape)
         ws = _workspace(lib.tm_cdt_workspace_size(batch, nd, shp), dev)
         st = lib.tm_cdt(_lib.ptr(input), _TORCH_TO_TM[input.dtype], batch, nd, shp,
@@ -325,7 +320,7 @@ def bfdt(input, metric="euclidean", sampling=None, return_distances=True, return
         ind = indices_out if indices_out is not None else torch.empty(
             (nd, *input.shape), dtype=torch.int32, device=dev)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         shp = _lib.i64_array(shape)
         ws = _workspace(lib.tm_bfdt_workspace_size(batch, nd, shp), dev)
         st = lib.tm_bfdt(_lib.ptr(input), _TORCH_TO_TM[input.dtype], batch, nd, shp,
@@ -370,7 +365,7 @@ def sinkhorn_fastiter(a, b, K, K_T, u, v, n_iter):
     _ot_check(K, d * d, "K")
     _ot_check(K_T, d * d, "K_T")
     lib = _lib.load()
-    with torch.cuda.device(u.device):
+    with _lib.on_device(u.device):
         ws = _iter_workspace(u.device)
         st = lib.tm_sinkhorn_fastiter(_lib.ptr(a), _lib.ptr(b), _lib.ptr(K), _lib.ptr(K_T),
                                       _lib.ptr(u), _lib.ptr(v), n, d, int(n_iter), _lib.ptr(ws),
@@ -389,7 +384,7 @@ def sinkhorn_logiter(log_a, log_b, M, M_T, log_u, log_v, n_iter, epsilon):
     _ot_check(M, d * d, "M")
     _ot_check(M_T, d * d, "M_T")
     lib = _lib.load()
-    with torch.cuda.device(log_u.device):
+    with _lib.on_device(log_u.device):
         ws = _iter_workspace(log_u.device)
         st = lib.tm_sinkhorn_logiter(_lib.ptr(log_a), _lib.ptr(log_b), _lib.ptr(M), _lib.ptr(M_T),
                                      _lib.ptr(log_u), _lib.ptr(log_v), n, d, int(n_iter),
@@ -423,7 +418,7 @@ def sinkhorn_f32_solve(a, b, cost_matrix, epsilon, max_iter, threshold=0.0, log_
     lib = _lib.load()
     dev = a.device
     check = int(check_every) if threshold > 0 else 0
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         nbytes = lib.tm_sinkhorn_f32_workspace_size(n, d, int(bool(log_space)), int(max_iter), check,
                                                     int(cost_matrix is None))
         ws = _workspace(nbytes, dev)
@@ -455,7 +450,7 @@ def sinkhorn_plan(log_u, log_v, cost_matrix, epsilon):
     """(n, d, d) transport plans exp((log u - C / eps) + log v), one pass."""
     n, d = _plan_args(log_u, log_v, cost_matrix, epsilon)
     out = torch.empty((n, d, d), dtype=torch.float32, device=log_u.device)
-    with torch.cuda.device(log_u.device):
+    with _lib.on_device(log_u.device):
         st = _lib.load().tm_sinkhorn_plan(_lib.ptr(log_u), _lib.ptr(log_v), _lib.ptr(cost_matrix), n, d,
                                           float(epsilon), _lib.ptr(out), _lib.stream_of(log_u.device))
     _lib.check(st, "sinkhorn_plan")
@@ -467,7 +462,7 @@ def sinkhorn_cost_grad(log_u, log_v, cost_matrix, epsilon, grad_distance):
     n, d = _plan_args(log_u, log_v, cost_matrix, epsilon)
     _ot_check(grad_distance, n, "grad_distance")
     out = torch.empty((d, d), dtype=torch.float32, device=log_u.device)
-    with torch.cuda.device(log_u.device):
+    with _lib.on_device(log_u.device):
         st = _lib.load().tm_sinkhorn_cost_grad(_lib.ptr(log_u), _lib.ptr(log_v), _lib.ptr(cost_matrix),
                                                _lib.ptr(grad_distance), n, d, float(epsilon),
                                                _lib.ptr(out), _lib.stream_of(log_u.device))
@@ -495,7 +490,7 @@ def sinkhorn_tc_solve(a, b, cost_matrix, epsilon, max_iter, threshold=0.0, check
     _ot_check(cost_matrix, d * d, "cost_matrix")
     lib = _lib.load()
     dev = a.device
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         stream = _lib.stream_of(dev)
         nbytes = lib.tm_sinkhorn_tc_workspace_size(n, d)
         ws = _workspace(nbytes, dev)

@@ -7,6 +7,7 @@ object is missing or fails to load, every operator raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 
@@ -28,7 +29,9 @@ I64P = ctypes.POINTER(ctypes.c_int64)
 F32P = ctypes.POINTER(ctypes.c_float)
 U8P = ctypes.POINTER(ctypes.c_uint8)
 
-# name -> (restype, argtypes); mirrors include/torchmorph_gb300.h
+# name -> (restype, argtypes); mirrors include/torchmorph_gb300.h.  load() binds the
+# host pointers (I64P, F32P, U8P) as void pointers, which take plain addresses as well as
+# ctypes arrays and pointers: an operator call then builds no pointer objects.
 SIGNATURES = {
     "tm_status_string": (ctypes.c_char_p, [c_int]),
     "tm_last_error": (ctypes.c_char_p, []),
@@ -171,7 +174,7 @@ def load():
             if fn is None:
                 continue
             fn.restype = res
-            fn.argtypes = args
+            fn.argtypes = [c_void if a in (I64P, F32P, U8P) else a for a in args]
         _lib = lib
     # install the autotuner's cached choices for this device (a missing or bad
     # cache leaves the built-in choices)
@@ -197,29 +200,64 @@ def check(status: int, what: str) -> None:
         raise TorchmorphError(status, f"{what}: {kind}: {msg}")
 
 
-def i64_array(values):
-    values = [int(v) for v in values]
+@functools.lru_cache(maxsize=4096)
+def _i64_cached(values):
     return (ctypes.c_int64 * max(1, len(values)))(*values)
 
 
-def f32_array(values):
-    values = [float(v) for v in values]
+@functools.lru_cache(maxsize=1024)
+def _f32_cached(values):
     return (ctypes.c_float * max(1, len(values)))(*values)
 
 
+def i64_array(values):
+    """const int64_t* of the values; short ones (shapes, origins) are built once and shared,
+    so nothing may write to them."""
+    values = tuple(map(int, values))
+    return _i64_cached(values) if len(values) <= 8 else (ctypes.c_int64 * len(values))(*values)
+
+
+def f32_array(values):
+    """const float* of the values, shared like i64_array's."""
+    values = tuple(map(float, values))
+    return _f32_cached(values) if len(values) <= 8 else (ctypes.c_float * len(values))(*values)
+
+
 def ctypes_f32(t: torch.Tensor):
-    """float* view of a contiguous float32 CPU tensor (kept alive by the caller)."""
-    return ctypes.cast(t.data_ptr(), F32P)
+    """Address of a contiguous float32 CPU tensor's data (kept alive by the caller)."""
+    return t.data_ptr()
 
 
 def ctypes_u8(t: torch.Tensor):
-    """uint8* view of a contiguous bool/uint8 CPU tensor (kept alive by the caller)."""
-    return ctypes.cast(t.data_ptr(), U8P)
+    """Address of a contiguous bool/uint8 CPU tensor's data (kept alive by the caller)."""
+    return t.data_ptr()
 
 
 def ptr(t: torch.Tensor | None):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
+
+
+class _NoGuard:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NO_GUARD = _NoGuard()
+
+
+def on_device(device: torch.device):
+    """A guard that makes `device` (of a CUDA tensor) current: nothing where it already is."""
+    return _NO_GUARD if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def stream_of(device: torch.device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """Handle of the current stream of a CUDA tensor's device."""
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
+    return torch.cuda.current_stream(device).cuda_stream

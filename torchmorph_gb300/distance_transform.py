@@ -47,7 +47,7 @@ def _prepare_distance_transform(input, return_distances, return_indices, distanc
 
 def _kernel_input(input: Tensor) -> Tensor:
     """Foreground carrier for the kernels: nonzero means foreground, as float32 in the reference."""
-    x = input.detach()
+    x = input.detach() if input.requires_grad else input
     if x.dtype in (torch.float32, torch.bool):
         return x.contiguous()
     if x.dtype == torch.uint8:

@@ -19,13 +19,19 @@ from .structure import _normalize_origin, _validate_origin, generate_binary_stru
 @functools.lru_cache(maxsize=None)
 def _default_structure(nd: int) -> Tensor:
     """The default element (cross, connectivity 1), built once per rank; read only."""
-    return generate_binary_structure(nd, 1)
+    return generate_binary_structure(nd, 1).contiguous()
 
 
-def _normalize_structure(structure: Tensor, spatial_ndim: int, name: str = "structure") -> Tensor:
+def _normalize_structure(structure: Tensor | None, spatial_ndim: int, name: str = "structure"):
+    """(CPU bool element, whether it is empty); None is the default cross."""
+    if structure is None:
+        return _default_structure(spatial_ndim), False
     if structure.ndim != spatial_ndim:
         raise ValueError(f"{name} dimension is not {spatial_ndim}, got {structure.ndim}")
-    return (structure != 0).detach().to(device="cpu", dtype=torch.bool).contiguous()
+    if structure.dtype != torch.bool or structure.device.type != "cpu":
+        structure = (structure != 0).detach().to(device="cpu", dtype=torch.bool)
+    structure = structure.contiguous()
+    return structure, not bool(structure.any())  # CPU tensor: no device sync
 
 
 def _binary_morphology_cuda_step(input, structure, border_value, origin, *, mode):
@@ -39,9 +45,7 @@ def _binary_morphology(input, structure, iterations, mask, output, border_value,
     until_stable = iterations < 1
     nd = validate_bcs_input(input)
     validate_output(input, output)
-    if structure is None:
-        structure = _default_structure(nd)
-    structure = _normalize_structure(structure, nd)
+    structure, empty = _normalize_structure(structure, nd)
     origin = _normalize_origin(origin, nd)
     _validate_origin(origin, structure)
     # foreground as bool (a bool input is used as is: comparing it with 0 is a slow
@@ -51,7 +55,6 @@ def _binary_morphology(input, structure, iterations, mask, output, border_value,
     if mask is not None and mask.shape != input.shape:
         raise ValueError(f"mask shape {mask.shape} must match input shape {input.shape}")
     mask_b = mask.to(device=input.device, dtype=torch.bool) if mask is not None else None
-    empty = not bool(structure.any())  # CPU tensor: no device sync
 
     def step(v):
         if empty:
@@ -131,14 +134,12 @@ def binary_hit_or_miss(input, structure1=None, structure2=None, output=None, ori
     validate_output(input, output)
     origin1 = _normalize_origin(origin1, nd)
     origin2 = origin1 if origin2 is None else _normalize_origin(origin2, nd)
-    if structure1 is None:
-        structure1 = generate_binary_structure(nd, 1)
-    structure1 = _normalize_structure(structure1, nd, "structure1")
+    structure1, _ = _normalize_structure(structure1, nd, "structure1")
     _validate_origin(origin1, structure1, "origin1")
     if structure2 is None:
         structure2 = torch.logical_not(structure1).contiguous()
     else:
-        structure2 = _normalize_structure(structure2, nd, "structure2")
+        structure2, _ = _normalize_structure(structure2, nd, "structure2")
     _validate_origin(origin2, structure2, "origin2")
     fg = input if input.dtype == torch.bool else input != 0
     if bool(structure1.any()):
@@ -164,12 +165,10 @@ def _one_pass(kind, input, structure, iterations, mask, output, border_value, or
     validate_output(input, output)
     if nd > 3:
         return None
-    if structure is None:
-        structure = _default_structure(nd)
-    structure = _normalize_structure(structure, nd)
+    structure, empty = _normalize_structure(structure, nd)
     origin = _normalize_origin(origin, nd)
     _validate_origin(origin, structure)
-    if not bool(structure.any()):
+    if empty:
         return None
     x = input if input.dtype == torch.bool and input.is_contiguous() else (input != 0).contiguous()
     res = _C.binary_composite(kind, x, structure, list(origin), bool(border_value))

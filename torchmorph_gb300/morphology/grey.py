@@ -6,6 +6,10 @@ operator for operator; the arithmetic runs in libtmcore through ``_C``.
 
 from __future__ import annotations
 
+import functools
+import math
+import operator
+
 import torch
 from torch import Tensor
 
@@ -27,9 +31,30 @@ def _element_kwargs(size, footprint, structure, mode, cval, origin) -> dict:
                 origin=origin)
 
 
+@functools.lru_cache(maxsize=256)
+def _small_box(size: tuple) -> Tensor:
+    return torch.zeros(size, dtype=torch.float32)
+
+
+def _box(size) -> Tensor:
+    """The flat box of a `size` argument; small ones are built once (read only)."""
+    size = tuple(map(operator.index, size))
+    return _small_box(size) if math.prod(size) <= 4096 else torch.zeros(size, dtype=torch.float32)
+
+
+_NO_FOOTPRINT = torch.empty(0, dtype=torch.bool)
+
+
+def _float_input(input: Tensor) -> Tensor:
+    """The kernels' input: `input` as a contiguous float32 tensor."""
+    if input.dtype == torch.float32 and input.is_contiguous() and not input.requires_grad:
+        return input
+    return input.detach().contiguous().float()
+
+
 def _resolve_element(spatial_ndim, size, footprint, structure):
     """(structure float32 CPU, footprint bool CPU or empty) with priority structure > footprint > size."""
-    fp_cpu = torch.empty(0, dtype=torch.bool)
+    fp_cpu = _NO_FOOTPRINT
     if structure is not None:
         struct = structure.to(torch.float32)
         if footprint is not None:
@@ -53,14 +78,16 @@ def _resolve_element(spatial_ndim, size, footprint, structure):
             size = (size,) * spatial_ndim
         if any(v <= 0 for v in size):
             raise ValueError("size values must be greater than zero")
-        struct = torch.zeros(tuple(size), dtype=torch.float32)
+        struct = _box(size)
     else:
         raise ValueError("At least one of size, footprint, or structure must be specified.")
     if struct.ndim != spatial_ndim:
         raise ValueError(
             f"Structure dimension {struct.ndim} must match spatial dimension {spatial_ndim}."
         )
-    return struct.detach().to(device="cpu", dtype=torch.float32).contiguous(), fp_cpu
+    if structure is not None:
+        struct = struct.detach().to(device="cpu", dtype=torch.float32).contiguous()
+    return struct, fp_cpu
 
 
 def _prepare(input, size, footprint, structure, mode, origin):
@@ -95,7 +122,7 @@ def _grey_morphology(
             raise ValueError("output= is not supported for a differentiable call")
         return result
     kernel = _C.grey_erosion_cuda if operation == "erosion" else _C.grey_dilation_cuda
-    result = kernel(input.detach().contiguous().float(), struct, fp, o, m, cval)
+    result = kernel(_float_input(input), struct, fp, o, m, cval)
     if output is not None:
         output.copy_(result)
         return output
@@ -110,7 +137,7 @@ class _GreyMorphologyFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, input, struct, fp, origin, mode, cval, dilation):
         kernel = _C.grey_dilation_arg if dilation else _C.grey_erosion_arg
-        out, arg = kernel(input.detach().contiguous().float(), struct, fp, origin, mode, cval)
+        out, arg = kernel(_float_input(input), struct, fp, origin, mode, cval)
         ctx.save_for_backward(arg)
         ctx.meta = (list(struct.shape), fp, origin, mode, dilation, input.dtype)
         return out
@@ -185,7 +212,7 @@ def _finish(result, output):
 def _one_pass(kind, input, size, footprint, structure, mode, cval, origin):
     """The one-pass 2-D composite kernel's result, or None outside its limits."""
     struct, fp, o, m = _prepare(input, size, footprint, structure, mode, origin)
-    return _C.grey_composite(kind, input.detach().contiguous().float(), struct, fp, o, m, cval)
+    return _C.grey_composite(kind, _float_input(input), struct, fp, o, m, cval)
 
 
 def morphological_gradient(input, size=None, footprint=None, structure=None, output=None,

@@ -54,7 +54,7 @@ def _solve(x, y, la, lb, nx, ny, eps, max_iter, threshold, check_every):
     g = torch.empty(y.shape[0], dtype=torch.float32, device=dev)
     cost = torch.empty(P, dtype=torch.float64, device=dev)
     its = torch.empty(P, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.tm_pointcloud_sinkhorn(
             _lib.ptr(x), _lib.ptr(y), _lib.ptr(la), _lib.ptr(lb), P, _lib.i64_array(nx),
             _lib.i64_array(ny), float(eps), int(max_iter), float(threshold), int(check_every),
@@ -71,7 +71,7 @@ def _grad(x, y, la, lb, f, g, nx, ny, eps, grad_cost, need_x, need_y):
     gx = torch.empty_like(x) if need_x else None
     gy = torch.empty_like(y) if need_y else None
     scale = grad_cost.to(device=dev, dtype=torch.float32).contiguous()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         _lib.check(lib.tm_pointcloud_sinkhorn_grad(
             _lib.ptr(x), _lib.ptr(y), _lib.ptr(la), _lib.ptr(lb), _lib.ptr(f), _lib.ptr(g), P,
             _lib.i64_array(nx), _lib.i64_array(ny), float(eps), _lib.ptr(scale), _lib.ptr(gx),

@@ -27,8 +27,9 @@ import torch
 from torch import Tensor
 
 from . import _lib
+from .morphology.binary import _normalize_structure
 from .morphology.grey import _MODE_MAP, _resolve_element
-from .morphology.structure import _normalize_origin, _validate_origin, generate_binary_structure
+from .morphology.structure import _normalize_origin, _validate_origin
 
 _TM_ERR_UNSUPPORTED = 2  # tm_status of a call outside a kernel's limits
 
@@ -114,7 +115,7 @@ class RaggedBatch:
             lib = _lib.load()
             n = len(self.shapes)
             dims = list(zip(*self.shapes))
-            with torch.cuda.device(self.data.device):
+            with _lib.on_device(self.data.device):
                 if self.ndim == 2:
                     nbytes = lib.tm_ragged_plan_size(n)
                     plan = torch.empty(int(nbytes), dtype=torch.uint8, device=self.data.device)
@@ -135,7 +136,16 @@ class RaggedBatch:
         """A batch with the same layout (and plan) over another buffer."""
         if data.shape != self.data.shape:
             raise ValueError("data must have the layout's buffer size")
-        return RaggedBatch(data, self.shapes, self.offsets, self._plan)
+        if not data.is_contiguous():
+            raise ValueError("RaggedBatch data must be a contiguous 1-D tensor")
+        # the layout was checked when this batch was made
+        batch = RaggedBatch.__new__(RaggedBatch)
+        batch.data = data
+        batch.shapes = list(self.shapes)
+        batch.offsets = list(self.offsets)
+        batch._plan = self._plan
+        batch._edt_plan = None
+        return batch
 
     def empty_like(self, dtype=None) -> "RaggedBatch":
         return self.with_data(torch.empty_like(self.data, dtype=dtype or self.data.dtype))
@@ -187,7 +197,7 @@ def _grey(name, batch, size, footprint, structure, mode, cval, origin, output):
     out = _output(batch, output, torch.float32)
     lib = _lib.load()
     fp_ptr = None if fp.numel() == 0 else _lib.ctypes_u8(fp)
-    with torch.cuda.device(batch.device):
+    with _lib.on_device(batch.device):
         _lib.check(getattr(lib, name)(_lib.ptr(batch.data), _lib.ptr(out.data), _lib.ptr(plan), plan.numel(),
                                       len(batch), _lib.ctypes_f32(struct), fp_ptr,
                                       _lib.i64_array(struct.shape), _lib.i64_array(o), _MODE_MAP[mode],
@@ -222,20 +232,16 @@ def _binary(name, batch, structure, border_value, origin, output):
     nd = batch.ndim
     if nd == 3:
         name = name.replace("tm_ragged_", "tm_ragged3d_")
-    if structure is None:
-        structure = generate_binary_structure(nd, 1)
-    if structure.ndim != nd:
-        raise ValueError(f"structure dimension is not {nd}, got {structure.ndim}")
-    st = (structure != 0).detach().to(device="cpu", dtype=torch.bool).contiguous()
+    st, empty = _normalize_structure(structure, nd)
     o = _normalize_origin(origin, nd)
     _validate_origin(o, st)
     plan = batch.plan
     out = _output(batch, output, torch.bool)
-    if not bool(st.any()):  # the reference's empty-structure result
+    if empty:  # the reference's empty-structure result
         out.data.fill_(name.endswith("erosion"))
         return out
     lib = _lib.load()
-    with torch.cuda.device(batch.device):
+    with _lib.on_device(batch.device):
         _lib.check(getattr(lib, name)(_lib.ptr(batch.data), _lib.ptr(out.data), _lib.ptr(plan), plan.numel(),
                                       len(batch), _lib.ctypes_u8(st), _lib.i64_array(st.shape),
                                       _lib.i64_array(o), int(bool(border_value)),
@@ -308,7 +314,7 @@ def euclidean_distance_transform(batch: RaggedBatch, return_distances: bool = Tr
     lib = _lib.load()
     n, nd, total = len(batch), batch.ndim, batch.data.numel()
     dev = batch.device
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         stream = _lib.stream_of(dev)
         plan = batch._edt_plan
         if plan is None:
