@@ -241,6 +241,50 @@ __device__ __forceinline__ float grad_pixel2d(const float *__restrict__ g, const
     return acc;
 }
 
+template <int K>
+struct FrameTaps {  // offsets of tap t = ky K + kx of a full K x K box: (dy[ky], dx[kx]); one value for all
+    int dy[K], dx[K];
+    float val;
+};
+
+// grad_pixel2d for a full box in the reflect, mirror and wrap modes, the same sums in the same
+// order.  They map at most two positions to a coordinate (but onto an axis of one), by way of
+// remainders: K ranges per axis instead of two for each of the K^2 taps, and the argument
+// bytes of a tap row loaded together.
+template <int K>
+__device__ __forceinline__ float grad_frame_pixel(const float *__restrict__ g, const uint8_t *__restrict__ a, int y, int x,
+                                                  const GradParams &p, const FrameTaps<K> &taps) {
+    const int H = p.shape[0], W = p.shape[1];
+    float acc = 0.f;
+    Ranges rx[K];
+#pragma unroll
+    for (int kx = 0; kx < K; kx++)
+        rx[kx] = preimage_ranges(x, W, p.mode, taps.dx[kx], taps.dx[kx] + W - 1);
+    for (int ky = 0; ky < K; ky++) {
+        const int dy = taps.dy[ky];
+        const Ranges ry = preimage_ranges(y, H, p.mode, dy, dy + H - 1);
+        const int64_t row0 = (int64_t)(ry.a0 - dy) * W, row1 = (int64_t)(ry.a1 - dy) * W;
+        const bool on0 = ry.b0 >= ry.a0, on1 = ry.b1 >= ry.a1;
+        bool hit[K][4];
+#pragma unroll
+        for (int kx = 0; kx < K; kx++) {
+            const int x0 = rx[kx].a0 - taps.dx[kx], x1 = rx[kx].a1 - taps.dx[kx];
+            const bool c0 = rx[kx].b0 >= rx[kx].a0, c1 = rx[kx].b1 >= rx[kx].a1;
+            const uint8_t t = (uint8_t)(ky * K + kx);
+            hit[kx][0] = on0 && c0 && a[row0 + x0] == t;
+            hit[kx][1] = on0 && c1 && a[row0 + x1] == t;
+            hit[kx][2] = on1 && c0 && a[row1 + x0] == t;
+            hit[kx][3] = on1 && c1 && a[row1 + x1] == t;
+        }
+#pragma unroll
+        for (int kx = 0; kx < K; kx++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)  // (about one hit per pixel in all)
+                if (hit[kx][i]) acc += g[(i & 2 ? row1 : row0) + (i & 1 ? rx[kx].a1 : rx[kx].a0) - taps.dx[kx]];
+    }
+    return acc;
+}
+
 __global__ void __launch_bounds__(kGradThreads) morph_grad_kernel(const float *__restrict__ gout,
                                                                   const uint8_t *__restrict__ arg,
                                                                   float *__restrict__ gin, GradParams p,
@@ -258,36 +302,67 @@ __global__ void __launch_bounds__(kGradThreads) morph_grad_kernel(const float *_
 
 // Frames of the float4 walkers (centred K x K flat boxes of 2-D items): the
 // outputs (forward) or input pixels (backward) outside the walkers'
-// rectangle, one thread each, with the per-voxel code above (same taps, same
-// order).  Launched behind the walker (programmatic dependent launch); each
+// rectangle, one thread each, with the per-voxel code's taps and order.
+// Launched behind the walker (programmatic dependent launch); each
 // finishes only once the walker has, so the stream's next work sees every
 // output.
-template <bool MAX>
+//
+// Bound: the latency of one pixel's border maps and dependent loads (a frame is a few
+// thousand pixels).  With the box compile-time, K row and K column maps instead of two per
+// tap, and the loads of a tap row together, 5 x 5, reflect: 64 x 128^2 forward 20.5 -> 10.3 us,
+// backward 52 -> 31 us; 8 x 512^2 18.5 -> 16.4 and 47 -> 33 us; 8 x 2048^2 115 -> 109 and
+// 174 -> 156 us.
+template <bool MAX, int K>
 __global__ void __launch_bounds__(256) arg_frame_kernel(const float *__restrict__ in, float *__restrict__ out,
                                                         uint8_t *__restrict__ arg, GradParams p,
-                                                        const __grid_constant__ GradTaps taps, vwalk::FrameRect fr) {
+                                                        const __grid_constant__ FrameTaps<K> taps,
+                                                        vwalk::FrameRect fr) {
     using Op = MorphOp<float, MAX>;
-    const int n = fr.count();
+    const int n = fr.count(), W = p.shape[1];
     for (int64_t item = blockIdx.y; item < p.batch; item += gridDim.y) {
         const float *src = in + item * p.numel_item;
         for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
             int y, x;
             fr.at(k, y, x);
+            int mx[K];
+#pragma unroll
+            for (int kx = 0; kx < K; kx++) mx[kx] = map_coord(x + taps.dx[kx], W, p.mode);
             float best = Op::identity();
             int a = kNoTap;
-            for (int t = 0; t < p.ntaps; t++) {
-                const int my = map_coord(y + taps.off[t][0], p.shape[0], p.mode);
-                const int mx = map_coord(x + taps.off[t][1], p.shape[1], p.mode);
-                const float v =
-                    Op::apply((my < 0 || mx < 0) ? p.cval : src[(int64_t)my * p.shape[1] + mx], taps.val[t]);
-                if (MAX ? v > best : v < best) {
-                    best = v;
-                    a = t;
-                }
+#pragma unroll
+            for (int ky = 0; ky < K; ky++) {
+                const int my = map_coord(y + taps.dy[ky], p.shape[0], p.mode);
+                float v[K];
+#pragma unroll
+                for (int kx = 0; kx < K; kx++)
+                    v[kx] = Op::apply((my < 0 || mx[kx] < 0) ? p.cval : src[(int64_t)my * W + mx[kx]], taps.val);
+#pragma unroll
+                for (int kx = 0; kx < K; kx++)
+                    if (MAX ? v[kx] > best : v[kx] < best) {
+                        best = v[kx];
+                        a = ky * K + kx;
+                    }
             }
-            const int64_t o = item * p.numel_item + (int64_t)y * p.shape[1] + x;
+            const int64_t o = item * p.numel_item + (int64_t)y * W + x;
             out[o] = best;
             arg[o] = (uint8_t)a;
+        }
+    }
+    pdl_wait();
+}
+
+template <int K>
+__global__ void __launch_bounds__(256, 4) grad_frame_two_kernel(const float *__restrict__ gout,
+                                                         const uint8_t *__restrict__ arg, float *__restrict__ gin,
+                                                         GradParams p, const __grid_constant__ FrameTaps<K> taps,
+                                                         vwalk::FrameRect fr) {
+    const int n = fr.count();
+    for (int64_t item = blockIdx.y; item < p.batch; item += gridDim.y) {
+        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+            int y, x;
+            fr.at(k, y, x);
+            gin[item * p.numel_item + (int64_t)y * p.shape[1] + x] =
+                grad_frame_pixel<K>(gout + item * p.numel_item, arg + item * p.numel_item, y, x, p, taps);
         }
     }
     pdl_wait();
@@ -307,6 +382,17 @@ __global__ void __launch_bounds__(256) grad_frame_kernel(const float *__restrict
         }
     }
     pdl_wait();
+}
+
+template <int K>
+FrameTaps<K> frame_taps(const GradTaps &taps) {
+    FrameTaps<K> f;
+    for (int k = 0; k < K; k++) {
+        f.dy[k] = taps.off[k * K][0];
+        f.dx[k] = taps.off[k][1];
+    }
+    f.val = taps.val[0];
+    return f;
 }
 
 // The walkers' box: a full centred K x K footprint (K 3 or 5) of a 2-D item
@@ -356,8 +442,12 @@ int run_arg_walk(const float *in, float *out, uint8_t *arg, const GradParams &p,
         kern<<<(unsigned)blocks, vwalk::kThreads, 0, s>>>(in, out, reinterpret_cast<uint32_t *>(arg), wp);
     TM_LAUNCH_CHECK("vwalk_arg_kernel");
     const vwalk::FrameRect fr{H, W, wp.ry0, wp.ry1, 4, W - 4};
-    TM_CHECK_CUDA(launch_pdl(arg_frame_kernel<MAX>, frame_grid(fr, p.batch), dim3(256), 0, s, in, out, arg, p, taps,
-                             fr));
+    if (k == 3)
+        TM_CHECK_CUDA(launch_pdl(arg_frame_kernel<MAX, 3>, frame_grid(fr, p.batch), dim3(256), 0, s, in, out, arg, p,
+                                 frame_taps<3>(taps), fr));
+    else
+        TM_CHECK_CUDA(launch_pdl(arg_frame_kernel<MAX, 5>, frame_grid(fr, p.batch), dim3(256), 0, s, in, out, arg, p,
+                                 frame_taps<5>(taps), fr));
     return TM_OK;
 }
 
@@ -391,8 +481,19 @@ int run_grad_walk(bool dilation, const float *gout, const uint8_t *arg, float *g
         kern<<<(unsigned)blocks, vwalk::kThreads, 0, s>>>(gout, reinterpret_cast<const uint32_t *>(arg), gin, wp);
     TM_LAUNCH_CHECK("vwalk_grad_kernel");
     const vwalk::FrameRect fr{H, W, wp.ry0, wp.ry1, 4, W - 4};
-    TM_CHECK_CUDA(
-        launch_pdl(grad_frame_kernel, frame_grid(fr, p.batch), dim3(256), 0, s, gout, arg, gin, p, taps, fr));
+    // Constant and nearest maps have no remainders to save, and the nearest edges hold longer
+    // ranges: 8 x 2048^2, 5 x 5, backward 150 us with the ranges of each tap, 153 with K per axis
+    // (reflect: 174 and 156; 64 x 128^2: 52 and 31).
+    const bool two = p.mode == TM_MODE_REFLECT || p.mode == TM_MODE_MIRROR || p.mode == TM_MODE_WRAP;
+    const dim3 grid = frame_grid(fr, p.batch);
+    if (!two || H < 2 || W < 2)
+        TM_CHECK_CUDA(launch_pdl(grad_frame_kernel, grid, dim3(256), 0, s, gout, arg, gin, p, taps, fr));
+    else if (k == 3)
+        TM_CHECK_CUDA(launch_pdl(grad_frame_two_kernel<3>, grid, dim3(256), 0, s, gout, arg, gin, p,
+                                 frame_taps<3>(taps), fr));
+    else
+        TM_CHECK_CUDA(launch_pdl(grad_frame_two_kernel<5>, grid, dim3(256), 0, s, gout, arg, gin, p,
+                                 frame_taps<5>(taps), fr));
     return TM_OK;
 }
 
