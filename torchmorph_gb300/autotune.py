@@ -3,11 +3,13 @@
 libtmcore keeps, for four operators, a table of implementation variants
 indexed by a work class (``tm_tune_*`` in include/torchmorph_gb300.h):
 
-* ``grey_flat2d``   flat 1-D / 2-D grey and binary boxes: TMA-staged
-  persistent tiles at full occupancy, plain loads one CTA per tile, or TMA
-  tiles with at most 1 / 2 CTAs per SM (class: log2 of the voxel count);
-* ``sinkhorn_f32``  FP32 Sinkhorn: 16 or 64 histogram pairs per tile, one or
-  two CTAs per SM (class from the pair count and the point count);
+* ``grey_flat2d``   flat 1-D / 2-D float boxes of 3 x 3 and 5 x 5 that the
+  register walkers do not take: TMA-staged persistent tiles at full occupancy,
+  plain loads one CTA per tile, or TMA tiles with at most 1 / 2 CTAs per SM
+  (class: log2 of the voxel count; other boxes have one implementation);
+* ``sinkhorn_f32``  FP32 Sinkhorn on matrices that do not stay in shared
+  memory: 16 or 64 histogram pairs per tile, one or two CTAs per SM (class
+  from the pair count and the point count);
 * ``edt_3d``        3-D exact EDT: bitmap shell search first, or the separable
   passes alone (class: log2 of the voxel count);
 * ``cdt_3d``        3-D chamfer distances: bitmap shell search first (persistent

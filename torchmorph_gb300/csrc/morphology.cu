@@ -10,14 +10,14 @@
 //
 // Kernels
 //   flat2d_kernel  -- flat rectangular footprints in 1-D/2-D: a shared-memory
-//                     tile with halo, separable row then column min/max.
-//                     Windows wider than kRun use the van Herk/Gil-Werman
-//                     split (shared middle block + register prefix/suffix
-//                     runs), so the cost per output stays ~2 reads.
-//   stencil_kernel -- everything else (non-flat values, arbitrary
-//                     footprints, 3..8-D): one thread per output, taps from
-//                     the launch parameters, an interior fast path with flat
-//                     offsets and a per-tap border path.
+//                     tile with halo, separable row then column min/max, in
+//                     van Herk/Gil-Werman runs (shared middle block + register
+//                     prefix/suffix runs) but for the narrowest windows.
+//   stencil_kernel -- 4..8-D and elements beyond the tile kernels: one thread
+//                     per output, taps from the launch parameters, an interior
+//                     fast path with flat offsets and a per-tap border path.
+// Binary 1-D to 3-D elements (boxes up to kBitBoxTaps voxels) run on bit-packed
+// tiles (bitmorph.cu, bitmorph3d.cu), other 3-D items on stencil3d.cu's tiles.
 #include <cmath>
 #include <cstring>
 #include <vector>
