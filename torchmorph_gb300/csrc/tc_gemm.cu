@@ -8,6 +8,7 @@ namespace tmc {
 namespace {
 
 struct StoreEpilogue {
+    static constexpr bool kEarlyA = false;  // (the caller's kernel before may write A)
     float *d;
     int64_t ldd;
     __device__ __forceinline__ void prefetch(int, int) const {}

@@ -131,12 +131,16 @@ struct Gemm3Smem {
     static_assert(STAGES * kStage >= 4 * kBN * 32 * 4, "the epilogue tile is staged in the operand ring");
 };
 
-// Epi: __device__ void operator()(const float *tile, int row, int n0) const,
+// Epi: __device__ void operator()(float *tile, int row, int n0) const,
 // called once by all 32 lanes of each accumulator warp together; lane l
 // owns output row `row` (32 consecutive rows per warp) and finds
 // D[row][n0 + c] at tile[c * 32 + l] (shared memory), c < kBN.
 // Epi::prefetch(row, n0) is called by the same threads when the mainloop
 // starts, to pull the epilogue's other inputs towards L2 early.
+//
+// Launched as a programmatic dependent: barriers, TMEM and, where Epi::kEarlyA
+// says that A was complete before the preceding kernel of the stream began, the
+// first k-blocks of A overlap that kernel; everything else waits for it.
 template <int STAGES, typename Epi>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm3_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
@@ -154,6 +158,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
     const int nk = K / kBK;
+    pdl_trigger();
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -176,14 +181,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         if (lane == 0) {
             bool ok = true;
             int issued = 0;
+            auto load_a = [&](int kb) {
+                const int s = kb % STAGES;
+                unsigned char *st = smem + s * L::kStage;
+                mbar_arrive_expect_tx(&full[s], L::kStage);
+                tma_load_2d(st, &ta_hi, kb * kBK, m0, &full[s]);
+                tma_load_2d(st + L::kTileA, &ta_lo, kb * kBK, m0, &full[s]);
+            };
+            const int early = Epi::kEarlyA ? min(nk, STAGES) : 0;
+            for (int kb = 0; kb < early; kb++) load_a(kb);
+            pdl_wait();
             for (int kb = 0; kb < nk && ok; kb++) {
                 const int s = kb % STAGES;
                 if (kb >= STAGES) ok = mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1, status);
                 if (!ok) break;
                 unsigned char *st = smem + s * L::kStage;
-                mbar_arrive_expect_tx(&full[s], L::kStage);
-                tma_load_2d(st, &ta_hi, kb * kBK, m0, &full[s]);
-                tma_load_2d(st + L::kTileA, &ta_lo, kb * kBK, m0, &full[s]);
+                if (kb >= early) load_a(kb);
                 tma_load_2d(st + 2 * L::kTileA, &tb_hi, kb * kBK, n0, &full[s]);
                 tma_load_2d(st + 2 * L::kTileA + L::kTileB, &tb_lo, kb * kBK, n0, &full[s]);
                 issued = kb + 1;
@@ -230,6 +243,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const int q = warp & 3;
         const uint32_t t_lane = tmem + ((uint32_t)(q * 32) << 16);
         const int row = m0 + q * 32 + lane;
+        pdl_wait();
         epi.prefetch(row, n0);
         float acc[kBN];
 #pragma unroll
@@ -306,7 +320,8 @@ int launch_gemm3(const void *a_hi, const void *a_lo, const void *b_hi, const voi
     auto kernel = gemm3_kernel<STAGES, Epi>;
     TM_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
     dim3 grid((unsigned)(N / kBN), (unsigned)(M / kBM));
-    kernel<<<grid, kGemmThreads, L::kBytes, stream>>>(ta_hi, ta_lo, tb_hi, tb_lo, (int)K, epi, status);
+    TM_CHECK_CUDA(launch_pdl(kernel, grid, dim3(kGemmThreads), L::kBytes, stream, ta_hi, ta_lo, tb_hi, tb_lo, (int)K, epi,
+                             status));
     TM_LAUNCH_CHECK("gemm3_kernel");
     return TM_OK;
 }
