@@ -307,7 +307,7 @@ def bench_ours(args, rank, world):
                      "traffic": load_traffic("edt"),
                      "scope": "whole EDT op (background bitmap + shell search; the separable passes "
                               "launch and exit for items the search finished), 17 algorithmic B/voxel"},
-        "gpu_launches": 4 * args.steps,
+        "gpu_launches": 5 * args.steps,
         "clocks": clk.summary(),
         "secondary": extra,
     }
@@ -736,7 +736,7 @@ def pointcloud_lines(dev, stream, cpu_baseline=True):
             "ex2_frac_of_nominal_all_active": round(2.0 * pairs / t_fixed / ex2_peak, 4),
             "rel_cost_error_vs_fp64": float(f"{rel:.3e}"),
             "marginal_l1_fp64_max": float(f"{marg:.3e}"), "fp64_problems_checked": 6,
-            "launches_per_solve": 5}
+            "launches_per_solve": 4}
     if cpu_baseline:
         cores = len(os.sched_getaffinity(0)) if hasattr(os, "sched_getaffinity") else os.cpu_count()
         t0 = time.perf_counter()

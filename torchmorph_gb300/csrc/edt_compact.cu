@@ -760,22 +760,17 @@ __global__ void __launch_bounds__(kShellThreads) edt_shell_kernel(const uint32_t
                 }
             }
         };
-        // inside large objects most voxels stay open: the warp leaves early, and the others at
-        // their next look (the rule of the straight-line search; 2 x 96 x 160 x 200, background
-        // 1 %: 189 -> 168 us with the passes that follow)
-        bool leave = false;
-#pragma unroll 1
-        for (int look = 0; look < 3 && !leave; look++) {
-            search(look == 0 ? 24 : look == 1 ? 64 : 128);
-            __syncwarp();
-            leave = __reduce_add_sync(~0u, __popc(U)) > (look == 0 ? 900 : look == 1 ? 600 : 256);
-            if (leave && (tid & 31) == 0) {
-                s_unresolved = 1;
-                atomicExch(&todo[item], 1);
-            }
-            leave = __any_sync(~0u, leave || *(volatile int *)&s_unresolved);
+        // inside large objects most voxels stay open: the warp leaves after 64 offsets, and so
+        // do those that look later (one of the straight-line search's three looks: each costs
+        // dense items; 2 x 96 x 160 x 200 with 1 % background, passes included: 189 -> 173 us)
+        search(64);
+        __syncwarp();
+        const bool most = __reduce_add_sync(~0u, __popc(U)) > 600;
+        if (most && (tid & 31) == 0) {
+            s_unresolved = 1;
+            atomicExch(&todo[item], 1);
         }
-        if (leave) break;
+        if (__any_sync(~0u, most || *(volatile int *)&s_unresolved)) break;
         search(kShellN);
         if (U) {
             s_unresolved = 1;
