@@ -223,14 +223,20 @@ def f32_array(values):
     return _f32_cached(values) if len(values) <= 8 else (ctypes.c_float * len(values))(*values)
 
 
+def _host_address(t: torch.Tensor) -> int:
+    if not t.is_cpu:  # libtmcore reads it on the host
+        raise RuntimeError("a structure or footprint must be a CPU tensor")
+    return t.data_ptr()
+
+
 def ctypes_f32(t: torch.Tensor):
     """Address of a contiguous float32 CPU tensor's data (kept alive by the caller)."""
-    return t.data_ptr()
+    return _host_address(t)
 
 
 def ctypes_u8(t: torch.Tensor):
     """Address of a contiguous bool/uint8 CPU tensor's data (kept alive by the caller)."""
-    return t.data_ptr()
+    return _host_address(t)
 
 
 def ptr(t: torch.Tensor | None):

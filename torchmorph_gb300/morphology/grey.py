@@ -6,7 +6,6 @@ operator for operator; the arithmetic runs in libtmcore through ``_C``.
 
 from __future__ import annotations
 
-import functools
 import math
 import operator
 
@@ -15,7 +14,7 @@ from torch import Tensor
 
 from .. import _C
 from .._validation import validate_bcs_input, validate_output
-from .structure import _normalize_origin, _validate_origin
+from .structure import _host_constant, _normalize_origin, _validate_origin
 
 _MODE_MAP = {
     "constant": 0,
@@ -31,18 +30,20 @@ def _element_kwargs(size, footprint, structure, mode, cval, origin) -> dict:
                 origin=origin)
 
 
-@functools.lru_cache(maxsize=256)
-def _small_box(size: tuple) -> Tensor:
-    return torch.zeros(size, dtype=torch.float32)
+def _host_zeros(size: tuple) -> Tensor:
+    """A flat element; the kernels' launchers read it on the host, whatever the default device."""
+    return torch.zeros(size, dtype=torch.float32, device="cpu")
 
 
 def _box(size) -> Tensor:
     """The flat box of a `size` argument; small ones are built once (read only)."""
     size = tuple(map(operator.index, size))
-    return _small_box(size) if math.prod(size) <= 4096 else torch.zeros(size, dtype=torch.float32)
+    if math.prod(size) > 4096:
+        return _host_zeros(size)
+    return _host_constant(size, lambda: _host_zeros(size))
 
 
-_NO_FOOTPRINT = torch.empty(0, dtype=torch.bool)
+_NO_FOOTPRINT = torch.empty(0, dtype=torch.bool, device="cpu")
 
 
 def _float_input(input: Tensor) -> Tensor:
@@ -71,7 +72,7 @@ def _resolve_element(spatial_ndim, size, footprint, structure):
         mask = footprint.to(torch.bool)
         if not mask.any():
             raise ValueError("All-zero footprint is not supported.")
-        struct = torch.zeros(tuple(mask.shape), dtype=torch.float32)
+        struct = _host_zeros(tuple(mask.shape))
         fp_cpu = mask.detach().to(device="cpu", dtype=torch.bool).contiguous()
     elif size is not None:
         if isinstance(size, int):

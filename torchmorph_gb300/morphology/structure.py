@@ -11,6 +11,21 @@ def _offset_grid(rank: int, radius: int, device=None) -> Tensor:
     return torch.stack(torch.meshgrid(*axes, indexing="ij"), dim=0)
 
 
+_HOST_CONSTANTS: dict = {}
+
+
+def _host_constant(key, make) -> Tensor:
+    """`make()`, a CPU tensor that nothing writes to, built once per `key`.  Kept only if it is a
+    plain tensor with memory of its own: one built under a fake-tensor or functional mode
+    belongs to that mode."""
+    t = _HOST_CONSTANTS.get(key)
+    if t is None:
+        t = make()
+        if type(t) is Tensor and t.data_ptr() != 0 and len(_HOST_CONSTANTS) < 256:
+            _HOST_CONSTANTS[key] = t
+    return t
+
+
 def generate_binary_structure(rank: int, connectivity: int) -> Tensor:
     """Boolean 3^rank element whose entries lie within `connectivity` unit steps of the centre."""
     if connectivity < 1 or connectivity > rank:
