@@ -6,7 +6,7 @@ import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
 from torchmorph_gb300 import _lib
-from torchmorph_gb300.morphology import grey
+from torchmorph_gb300.morphology import binary, generate_binary_structure, grey
 
 
 def _is_plain(t):
@@ -46,3 +46,18 @@ def test_no_host_address_of_a_device_tensor():
         _lib.ctypes_f32(torch.zeros(3, device="meta"))
     with pytest.raises(RuntimeError, match="CPU tensor"):
         _lib.ctypes_u8(torch.zeros(3, dtype=torch.bool, device="meta"))
+
+
+@pytest.mark.parametrize("nd", [1, 2, 3, 4])
+def test_default_cross_under_a_default_device(nd):
+    with torch.device("meta"):
+        inside, empty = binary._normalize_structure(None, nd)
+    after, _ = binary._normalize_structure(None, nd)
+    assert not empty and _is_plain(inside) and _is_plain(after)
+    assert torch.equal(after, generate_binary_structure(nd, 1))
+
+
+def test_default_cross_made_under_a_mode_is_not_kept():
+    with FakeTensorMode():
+        binary._normalize_structure(None, 5)
+    assert _is_plain(binary._normalize_structure(None, 5)[0])

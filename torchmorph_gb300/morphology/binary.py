@@ -6,20 +6,17 @@ dilation step is one libtmcore launch through ``_C``.
 
 from __future__ import annotations
 
-import functools
-
 import torch
 from torch import Tensor
 
 from .. import _C
 from .._validation import validate_bcs_input, validate_output
-from .structure import _normalize_origin, _validate_origin, generate_binary_structure
+from .structure import _host_constant, _normalize_origin, _offset_grid, _validate_origin
 
 
-@functools.lru_cache(maxsize=None)
 def _default_structure(nd: int) -> Tensor:
-    """The default element (cross, connectivity 1), built once per rank; read only."""
-    return generate_binary_structure(nd, 1).contiguous()
+    """The default element (cross, connectivity 1) on the CPU, built once per rank; read only."""
+    return _host_constant(("cross", nd), lambda: ((_offset_grid(nd, 1, "cpu") != 0).sum(dim=0) <= 1).contiguous())
 
 
 def _normalize_structure(structure: Tensor | None, spatial_ndim: int, name: str = "structure"):
