@@ -443,14 +443,12 @@ int launch_edt(const In *in, const Geometry &g, const float *sampling, EdtOutput
         } else if (p.L <= kSmemStackMaxL) {
             size_t smem = (size_t)kEdtThreads * p.L * sizeof(int16_t);
             if (final_pass) {
-                if (smem > 48 * 1024)
-                    TM_CHECK_CUDA(cudaFuncSetAttribute(edt_envelope_smem_kernel<V, true>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                const int st = allow_shared_memory((const void *)edt_envelope_smem_kernel<V, true>, smem);
+                if (st != TM_OK) return st;
                 edt_envelope_smem_kernel<V, true><<<blocks, kEdtThreads, smem, stream>>>(gin, fin, gout, fout, p, o);
             } else {
-                if (smem > 48 * 1024)
-                    TM_CHECK_CUDA(cudaFuncSetAttribute(edt_envelope_smem_kernel<V, false>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                const int st = allow_shared_memory((const void *)edt_envelope_smem_kernel<V, false>, smem);
+                if (st != TM_OK) return st;
                 edt_envelope_smem_kernel<V, false><<<blocks, kEdtThreads, smem, stream>>>(gin, fin, gout, fout, p, o);
             }
             TM_LAUNCH_CHECK("edt_envelope_smem_kernel");

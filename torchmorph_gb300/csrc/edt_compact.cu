@@ -1637,9 +1637,8 @@ int launch_lines(const void *src, int32_t *c2, float *dist, int32_t *indices, in
     const int64_t tiles = p.batch * (MODE == 1 ? (int64_t)p.L0 * ceil_div(p.L2, NL) : ceil_div(rows, NL));
     if (tiles >= ((int64_t)1 << 31)) return fail(TM_ERR_TOO_LARGE, "too many blocks");
     const size_t smem = line_tile(NL, L).total;
-    if (smem > 48 * 1024)
-        TM_CHECK_CUDA(cudaFuncSetAttribute(edt_line_kernel<MODE, NL, T, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
+    const int st = allow_shared_memory((const void *)edt_line_kernel<MODE, NL, T, OUT>, smem);
+    if (st != TM_OK) return st;
     const int64_t grid = todo ? std::min<int64_t>(tiles, wave_ctas(edt_line_kernel<MODE, NL, T, OUT>, T, smem)) : tiles;
     TM_CHECK_CUDA(launch_pdl(edt_line_kernel<MODE, NL, T, OUT>, dim3((unsigned)grid), dim3(T), smem, stream, src, c2,
                              dist, indices, sqdist, p, todo));
@@ -1661,8 +1660,8 @@ int launch_bits0(const In *in, int16_t *c1, const CompactParams &p, const int *t
     const dim3 threads(32 * wpc, groups);
     const size_t smem = (size_t)nw * cols * groups * 4;
     auto go = [&](auto kernel) -> int {
-        if (smem > 48 * 1024)
-            TM_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const int st = allow_shared_memory((const void *)kernel, smem);
+        if (st != TM_OK) return st;
         if (todo) {  // overlaps the shell search's last CTAs
             const int64_t grid = std::min<int64_t>(blocks, wave_ctas(kernel, 32 * wpc * groups, smem));
             TM_CHECK_CUDA(launch_pdl(kernel, dim3((unsigned)grid), threads, smem, stream, in, c1, p, todo));
@@ -1757,9 +1756,7 @@ int edt_compact_run(const void *input, int in_dtype, const Geometry &g, const Ed
         if (ww == 4) {  // rows of 97..128 voxels: straight-line search
             if ((st = launch_ct(edt_shell_ct_kernel<4>)) != TM_OK) return st;
         } else {
-            if (sm.total > 48 * 1024)
-                TM_CHECK_CUDA(cudaFuncSetAttribute(edt_shell_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)sm.total));
+            if ((st = allow_shared_memory((const void *)edt_shell_kernel, sm.total)) != TM_OK) return st;
             edt_shell_kernel<<<(unsigned)sblocks, kShellThreads, sm.total, stream>>>(bm, dist, indices, sqdist, todo,
                                                                                     p);
         }
@@ -1897,8 +1894,7 @@ int ragged_edt3_run(const void *input, int in_f32, const ReItem *items, int nite
     int dev = 0;
     TM_CHECK_CUDA(cudaGetDevice(&dev));
     if (cached_dev != dev || cached_smem != smem) {
-        TM_CHECK_CUDA(cudaFuncSetAttribute(ragged_edt3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)c12_smem(kRaggedC12MaxLine, kRaggedC12MaxLine).total));
+        if ((st = allow_shared_memory((const void *)ragged_edt3_kernel, smem)) != TM_OK) return st;
         TM_CHECK_CUDA(
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cached_per_sm, ragged_edt3_kernel, kC12Threads, smem));
         cached_dev = dev;

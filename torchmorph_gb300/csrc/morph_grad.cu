@@ -951,8 +951,7 @@ int run_arg(const float *in, float *out, uint8_t *arg, int64_t batch, int ndim, 
         const int P = pitch2d(tp.ext_x);
         const size_t smem = (size_t)(kT2H + tp.ext_y) * P * sizeof(float);
         auto kern = P == 136 ? morph_arg2d_kernel<MAX, 136> : morph_arg2d_kernel<MAX, 160>;
-        if (smem > 48 * 1024)
-            TM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if ((st = allow_shared_memory((const void *)kern, smem)) != TM_OK) return st;
         kern<<<grid2d(p), kT2Threads, smem, s>>>(in, out, arg, p, tp);
         TM_LAUNCH_CHECK("morph_arg2d_kernel");
         return TM_OK;
@@ -981,8 +980,7 @@ int run_grad(bool dilation, const float *gout, const uint8_t *arg, float *gin, i
         const int P = pitch2d(tp.ext_x);
         const size_t smem = (size_t)(kT2H + tp.ext_y) * P * sizeof(uint2);
         auto kern = P == 136 ? morph_grad2d_kernel<136> : morph_grad2d_kernel<160>;
-        if (smem > 48 * 1024)
-            TM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if ((st = allow_shared_memory((const void *)kern, smem)) != TM_OK) return st;
         kern<<<grid2d(p), kT2Threads, smem, s>>>(gout, arg, gin, p, taps, tp);
         TM_LAUNCH_CHECK("morph_grad2d_kernel");
         return TM_OK;
@@ -1072,15 +1070,13 @@ int run_composite(int op, const float *in, float *out, int64_t batch, int ndim, 
     else
         kern = op == 0 ? (P == 136 ? grey_composite2d_kernel<0, 136, false> : grey_composite2d_kernel<0, 160, false>)
                        : (P == 136 ? grey_composite2d_kernel<1, 136, false> : grey_composite2d_kernel<1, 160, false>);
-    cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) {
+    st = allow_shared_memory((const void *)kern, smem);
+    if (st == TM_OK) {
         kern<<<grid2d(pd), kT2Threads, smem, s>>>(in, out, pd, *tp);
-        e = cudaGetLastError();
+        st = launch_check("grey_composite2d_kernel");
     }
     delete tp;
-    TM_CHECK_CUDA(e);
-    return TM_OK;
+    return st;
 }
 
 }  // namespace

@@ -342,8 +342,7 @@ int launch_flat2d_small(const T *in, T *out, Flat2DParams p, int64_t batch, int 
     int dev = 0;
     TM_CHECK_CUDA(cudaGetDevice(&dev));
     if (cached_smem != tsmem || cached_dev != dev) {
-        TM_CHECK_CUDA(cudaFuncSetAttribute(flat2d_tma_kernel<T, MAX, KH, KW>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
+        if ((st = allow_shared_memory((const void *)flat2d_tma_kernel<T, MAX, KH, KW>, tsmem)) != TM_OK) return st;
         int per_sm = 0;
         TM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, flat2d_tma_kernel<T, MAX, KH, KW>,
                                                                     kFlatThreads, tsmem));
@@ -364,9 +363,8 @@ int launch_flat2d(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, c
     const int RH = kTileH + p.kh - 1, RWp = stage_pitch(p.kw);
     const size_t rows_bytes = KH == 0 ? (size_t)RH * kRowsPitch * sizeof(T) : 0;
     const size_t smem = (size_t)RH * RWp * sizeof(T) + rows_bytes;
-    if (smem > 48 * 1024)
-        TM_CHECK_CUDA(cudaFuncSetAttribute(flat2d_kernel<T, MAX, KH, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
+    const int st = allow_shared_memory((const void *)flat2d_kernel<T, MAX, KH, KW>, smem);
+    if (st != TM_OK) return st;
     dim3 grid((unsigned)ceil_div(p.W, kTileW), (unsigned)ceil_div(p.H, kTileH),
               (unsigned)(batch < 65535 ? batch : 65535));
     // windows of a runtime size: their row pass wants an odd row pitch, which a TMA box

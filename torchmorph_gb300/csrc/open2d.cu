@@ -477,8 +477,7 @@ int run_open2d(const float *in, float *out, int64_t batch, int ndim, const int64
     p.d_cols1 = make_fastdiv(kOTileW + p.kw - 1);
     const size_t smem = open2d_smem(p.kh, p.kw);
     auto kernel = open2d_kernel<MAX1, TOPHAT>;
-    if (smem > 48 * 1024)
-        TM_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if ((st = allow_shared_memory((const void *)kernel, smem)) != TM_OK) return st;
     const int64_t ring = (int64_t)tiles_x * tiles_y - (int64_t)(p.tr1 - p.tr0) * (p.tc1 - p.tc0);
     const int64_t tiles = batch * ring;
     if (tiles >= ((int64_t)1 << 31)) return fail(TM_ERR_TOO_LARGE, "too many tiles");

@@ -189,8 +189,6 @@ int persistent_grid(K kernel, size_t smem, int *grid) {
                 return TM_OK;
             }
     }
-    // the attribute allows the largest tile on the device (minus the kernel's static
-    // shared memory), so that a later launch with a larger tile than a cached one fits
     int optin = 0;
     TM_CHECK_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cudaFuncAttributes fa;
@@ -198,7 +196,8 @@ int persistent_grid(K kernel, size_t smem, int *grid) {
     const int max_dynamic = optin - (int)fa.sharedSizeBytes;
     if (smem > (size_t)max_dynamic)
         return fail(TM_ERR_UNSUPPORTED, "ragged tile needs %zu bytes of shared memory", smem);
-    TM_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic));
+    const int st = allow_shared_memory((const void *)kernel, smem);
+    if (st != TM_OK) return st;
     int per_sm = 0;
     TM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kFlatThreads, smem));
     if (per_sm < 1) return fail(TM_ERR_UNSUPPORTED, "ragged tile does not fit on an SM");

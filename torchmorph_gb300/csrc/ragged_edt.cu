@@ -390,8 +390,7 @@ extern "C" int tm_ragged_edt(const void *input, int in_dtype, const void *plan, 
     int dev = 0;
     TM_CHECK_CUDA(cudaGetDevice(&dev));
     if (cached_dev != dev || cached_smem != smem) {
-        TM_CHECK_CUDA(cudaFuncSetAttribute(ragged_edt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)((size_t)kReSmemL * kReThreads * sizeof(int16_t))));
+        if ((st = allow_shared_memory((const void *)ragged_edt_kernel, smem)) != TM_OK) return st;
         TM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cached_per_sm, ragged_edt_kernel, kReThreads,
                                                                     smem));
         cached_dev = dev;

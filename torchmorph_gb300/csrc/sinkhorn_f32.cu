@@ -990,13 +990,13 @@ int cluster_count(int ctas) {
         cudaLaunchAttribute attr{};
         cudaLaunchConfig_t cfg = cluster_config(ctas, ctas, kClMaxSmem - 2048, nullptr, &attr);
         int n = 0;
-        const bool ok =
-            cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) ==
-                cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess;
-        if (!ok) cudaGetLastError();
-        c = ok && n > 0 ? n : -1;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            allow_shared_memory(kern, cfg.dynamicSmemBytes) != TM_OK ||
+            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;  // (not kept: the next call asks again)
+        }
+        c = n > 0 ? n : -1;
         cached[dev][ctas].store(c, std::memory_order_relaxed);
     }
     return c > 0 ? c : 0;
@@ -1377,7 +1377,8 @@ bool sk_slab_launch(SkArgs &A, cudaStream_t s, int *st) {
     if (!slab_shape<LOG, V>(A.n, A.d, std::min(sm_count(), kSlabMaxCtas), &sh)) return false;
     const void *kern = (const void *)sk_slab_kernel<LOG, V>;
     auto run = [&]() -> int {
-        TM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+        const int ready = allow_shared_memory(kern, sh.smem);
+        if (ready != TM_OK) return ready;
         TM_CHECK_CUDA(cudaMemsetAsync(A.ctl, 0, sizeof(SkControl), s));
         void *params[] = {&A, &sh};
         TM_CHECK_CUDA(cudaLaunchCooperativeKernel(kern, dim3(sh.ctas * sh.groups), dim3(kSkThreads), params, sh.smem, s));
@@ -1400,7 +1401,8 @@ bool sk_cluster(bool log_form, const SkArgs &A, cudaStream_t s, int *st) {
     if (log_form || !A.paired || !cluster_shape(A.n, A.d, &sh)) return false;
     auto run = [&](auto kernel) -> int {
         TM_CHECK_CUDA(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        TM_CHECK_CUDA(cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+        const int ready = allow_shared_memory((const void *)kernel, sh.smem);
+        if (ready != TM_OK) return ready;
         TM_CHECK_CUDA(cudaMemsetAsync(A.ctl, 0, sizeof(SkControl), s));
         cudaLaunchAttribute attr[2]{};
         cudaLaunchConfig_t cfg = cluster_config(sh.ctas, sh.clusters * sh.ctas, sh.smem, s, attr);

@@ -282,7 +282,8 @@ int grid_for_kernel(size_t smem, int *grid) {
             return TM_OK;
         }
     auto kernel = stencil3d_kernel<T, MAX, SEP>;
-    TM_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStencil3Smem));
+    const int st = allow_shared_memory((const void *)kernel, smem);
+    if (st != TM_OK) return st;
     int per_sm = 0;
     TM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kT3Threads, smem));
     if (per_sm < 1) return fail(TM_ERR_UNSUPPORTED, "3-D tile does not fit on an SM");

@@ -318,7 +318,7 @@ int launch_gemm3(const void *a_hi, const void *a_lo, const void *b_hi, const voi
     st = device_status_word(&status);
     if (st != TM_OK) return st;
     auto kernel = gemm3_kernel<STAGES, Epi>;
-    TM_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
+    if ((st = allow_shared_memory((const void *)kernel, L::kBytes)) != TM_OK) return st;
     dim3 grid((unsigned)(N / kBN), (unsigned)(M / kBM));
     TM_CHECK_CUDA(launch_pdl(kernel, grid, dim3(kGemmThreads), L::kBytes, stream, ta_hi, ta_lo, tb_hi, tb_lo, (int)K, epi,
                              status));

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <unordered_map>
 
 #include "tm_common.cuh"
 #include "tm_tma.cuh"
@@ -44,6 +45,26 @@ int sm_count() {
         cached[dev] = n;
     }
     return cached[dev];
+}
+
+int allow_shared_memory(const void *kernel, size_t smem) {
+    if (smem <= 32 * 1024) return TM_OK;  // (with the static part within the default limit)
+    static std::mutex mu;
+    static std::unordered_map<const void *, uint64_t> raised;  // kernel -> devices
+    int dev = 0;
+    TM_CHECK_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(TM_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
+    std::lock_guard<std::mutex> lock(mu);
+    uint64_t &devices = raised[kernel];
+    if (devices >> dev & 1) return TM_OK;
+    int optin = 0;
+    TM_CHECK_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes fa;
+    TM_CHECK_CUDA(cudaFuncGetAttributes(&fa, kernel));
+    TM_CHECK_CUDA(
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    devices |= 1ull << dev;
+    return TM_OK;
 }
 
 int make_geometry(int64_t batch, int ndim, const int64_t *shape, Geometry *g) {

@@ -26,6 +26,12 @@ inline int launch_check(const char *kernel) { return cuda_check(cudaGetLastError
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+// Lets launches of `kernel` take `smem` bytes of dynamic shared memory.  The limit is an
+// attribute that all threads of the process share, so it is raised to the most the device
+// gives the kernel, once per kernel and device: set to each call's own size, one thread's
+// smaller size could come between another's setting and its launch.
+int allow_shared_memory(const void *kernel, size_t smem);
+
 // Implementation variants picked by the autotuner (tm_tune_set), per operator
 // and work class; -1 = the library's built-in choice.  Every variant of an
 // operator gives bit-identical results.
