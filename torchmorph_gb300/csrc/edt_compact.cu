@@ -52,6 +52,7 @@ struct CompactParams {
     int64_t numel_item;
     uint32_t w0, w1, w2;  // squared voxel sizes of the axes in units of unit2 (1 for unit spacing)
     float unit2;          // a power of 4
+    FastDiv d_l1, d_line;  // line passes: rows of a plane, positions of a line
 };
 
 // floor(sqrt(u)) for 0 <= u < 2^31 (the float estimate is off by at most one).
@@ -1629,18 +1630,20 @@ namespace {
 
 // One pass over the lines: a resident wave striding over the tiles where items may be
 // finished already (todo), else a CTA per tile.
-template <int MODE, int NL, int T, int OUT>
-int launch_lines(const void *src, int32_t *c2, float *dist, int32_t *indices, int32_t *sqdist, const CompactParams &p,
+template <int MODE, int NL, int T, int OUT, bool FLAT = false>
+int launch_lines(const void *src, int32_t *c2, float *dist, int32_t *indices, int32_t *sqdist, CompactParams p,
                  const int *todo, cudaStream_t stream) {
     const int L = MODE == 2 ? p.L2 : p.L1;
     const int64_t rows = MODE == 0 ? p.L0 : (int64_t)p.L0 * p.L1;
     const int64_t tiles = p.batch * (MODE == 1 ? (int64_t)p.L0 * ceil_div(p.L2, NL) : ceil_div(rows, NL));
     if (tiles >= ((int64_t)1 << 31)) return fail(TM_ERR_TOO_LARGE, "too many blocks");
+    p.d_l1 = make_fastdiv((uint32_t)p.L1);
+    p.d_line = make_fastdiv((uint32_t)L);
     const size_t smem = line_tile(NL, L).total;
-    const int st = allow_shared_memory((const void *)edt_line_kernel<MODE, NL, T, OUT>, smem);
+    const int st = allow_shared_memory((const void *)edt_line_kernel<MODE, NL, T, OUT, FLAT>, smem);
     if (st != TM_OK) return st;
-    const int64_t grid = todo ? std::min<int64_t>(tiles, wave_ctas(edt_line_kernel<MODE, NL, T, OUT>, T, smem)) : tiles;
-    TM_CHECK_CUDA(launch_pdl(edt_line_kernel<MODE, NL, T, OUT>, dim3((unsigned)grid), dim3(T), smem, stream, src, c2,
+    const int64_t grid = todo ? std::min<int64_t>(tiles, wave_ctas(edt_line_kernel<MODE, NL, T, OUT, FLAT>, T, smem)) : tiles;
+    TM_CHECK_CUDA(launch_pdl(edt_line_kernel<MODE, NL, T, OUT, FLAT>, dim3((unsigned)grid), dim3(T), smem, stream, src, c2,
                              dist, indices, sqdist, p, todo));
     TM_LAUNCH_CHECK("edt_line_kernel");
     return TM_OK;
@@ -1650,9 +1653,10 @@ template <typename In>
 int launch_bits0(const In *in, int16_t *c1, const CompactParams &p, const int *todo, cudaStream_t stream) {
     const int64_t inner = p.numel_item / p.L0;
     const int nw = (p.L0 + 31) / 32, wpc = std::min(nw, kBitsWarps);
-    // 4 columns per lane once they fill the device (a warp per 32 rows and 128 columns)
+    // 4 columns per lane once they give every SM 8 warps (a warp per 32 rows and 128 columns):
+    // 2 x 88 x 180 x 214 19 -> 11.5 us, 64 x 250 x 512 20 -> 14; at half as many 16 x 512^2 11 -> 14
     const bool wide = inner % 4 == 0 && ((uintptr_t)in & (4 * sizeof(In) - 1)) == 0 &&
-                      p.batch * (inner / 128) * nw >= (int64_t)sm_count() * 32;
+                      p.batch * (inner / 128) * nw >= (int64_t)sm_count() * 8;
     const int cols = wide ? 128 : 32;
     const int groups = (int)std::max<int64_t>(1, std::min<int64_t>(kBitsWarps / wpc, ceil_div(inner, cols)));
     const int64_t blocks = p.batch * ceil_div(inner, (int64_t)cols * groups);
@@ -1769,8 +1773,19 @@ int edt_compact_run(const void *input, int in_dtype, const Geometry &g, const Ed
     // lines (68 KB at 1333 voxels) leave room for few CTAs
     auto rows = [&](auto mode, auto out, const void *src, int L) -> int {
         constexpr int M = decltype(mode)::value, O = decltype(out)::value;
-        if (L <= kShortLine) return launch_lines<M, 32, 256, O>(src, nullptr, dist, indices, sqdist, p, todo, stream);
-        if (L <= kMediumLine) return launch_lines<M, 8, 256, O>(src, nullptr, dist, indices, sqdist, p, todo, stream);
+        // flat where units of 128 would idle for a third of their positions: rows of 130, 80, 63
+        // voxels gain 8, 4, 14 %, rows of 100 nothing, 202 lose 4 %
+        const bool flat = ceil_div(L, 128) * 128 * 2 > 3 * (int64_t)L;
+        // (whether tiles of n lines still give every SM a few)
+        auto fills = [&](int n) { return p.batch * ceil_div(M == 2 ? (int64_t)p.L0 * p.L1 : p.L0, n) >= 4 * (int64_t)sm_count(); };
+        auto go = [&](auto lines) -> int {
+            constexpr int NL = decltype(lines)::value;
+            return flat ? launch_lines<M, NL, 256, O, true>(src, nullptr, dist, indices, sqdist, p, todo, stream)
+                        : launch_lines<M, NL, 256, O, false>(src, nullptr, dist, indices, sqdist, p, todo, stream);
+        };
+        if (L <= kShortLine && fills(32)) return go(std::integral_constant<int, 32>());
+        if (L <= kShortLine || (M == 2 && L <= 2 * kShortLine && fills(16))) return go(std::integral_constant<int, 16>());
+        if (L <= kMediumLine) return go(std::integral_constant<int, 8>());
         return launch_lines<M, 8, 512, O>(src, nullptr, dist, indices, sqdist, p, todo, stream);
     };
     const std::integral_constant<int, 0> k0;

@@ -31,6 +31,16 @@
 // 272 us, Bernoulli(0.99) 623 -> 250 us.  Windows decided per warp instead of by lists
 // (a warp runs the widest ring any of its lanes needs) took 138 us on the 2-D masks;
 // open positions walked inside their group's thread 121 us.
+//
+// Dense backgrounds take the first window alone, and there the instructions around it count:
+// a tile without an open group skips the lists and reads its distances, all below the window's
+// bound, from a table.  FLAT tiles (modes 0 and 2) stage and write their lines, adjacent rows,
+// as one run of positions, the others in units of 128 positions of a line: the flat form
+// divides by the line length for every position, the units idle in a line's last one.
+// Bernoulli(0.5), distances alone, one thread or warp per line -> units and lists for all ->
+// now: 64 x 256^2 21.3 -> 28.1 -> 25.4 us, 64 x 250 x 512 (3-D) 32.0 -> 48.6 -> 38.1, 4 x 128
+// x 128 x 130 91.5 -> 117.7 -> 85.9 (units there 93.6), 8 x 64 x 64 x 63 30.6 -> 32.7 -> 25.9;
+// 64 x 128^2 11.1 -> 15.6 -> 12.5 (tiles of 16 lines; of 32: 14.4).
 constexpr int kLineQ = 8;        // positions per thread and window step
 constexpr int kLineK1 = 4;       // window radii
 constexpr int kLineK2 = 12;
@@ -211,7 +221,7 @@ __device__ __forceinline__ void line_ring(const uint32_t *g, const uint32_t *c, 
     }
 }
 
-template <int MODE, int NL, int T, int OUT>
+template <int MODE, int NL, int T, int OUT, bool FLAT>
 __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__restrict__ src, int32_t *__restrict__ c2,
                                                                 float *__restrict__ dist,
                                                                 int32_t *__restrict__ indices,
@@ -221,7 +231,7 @@ __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__res
     constexpr int kSlots = T / NL;
     // list entries: line and group of 8 positions, line and position (32 lines reach 1024
     // positions, 8 reach 4096)
-    constexpr int kPosBits = NL == 32 ? 10 : 12, kPosMask = (1 << kPosBits) - 1;
+    constexpr int kPosBits = NL == 32 ? 10 : (NL == 16 ? 11 : 12), kPosMask = (1 << kPosBits) - 1;
     constexpr int kTaskBits = kPosBits - 3, kTaskMask = (1 << kTaskBits) - 1;
     const int L = MODE == 2 ? p.L2 : p.L1;
     const LineTile tl = line_tile(NL, L);
@@ -237,6 +247,9 @@ __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__res
     const int tiles_x = MODE == 1 ? (W + NL - 1) / NL : 1;
     const int rows = MODE == 0 ? p.L0 : p.L0 * p.L1;
     const int64_t tiles = MODE == 1 ? (int64_t)p.L0 * tiles_x : (rows + NL - 1) / NL;
+    __shared__ float root[kSqrtTab];  // distances of small values (barriers follow)
+    __shared__ int at[NL];            // FLAT, mode 2: z << 16 | y of a line
+    if (MODE != 1 && tid < kSqrtTab) root[tid] = line_dist(tid, p.unit2);
     const uint32_t weight = MODE == 2 ? p.w2 : p.w1, w0 = p.w0, w1 = p.w1;
     const float inv_weight = 1.0f / (float)weight;
     const uint32_t far_limit = min(weight * (uint32_t)(kLineFar * kLineFar), kBig);
@@ -263,7 +276,13 @@ __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__res
             const int f0 = (int16_t)(f & 0xffff), f1 = f >> 16;
             return f0 < 0 ? kBig : w0 * (uint32_t)((z - f0) * (z - f0)) + w1 * (uint32_t)((y - f1) * (y - f1));
         };
-        if (tid < NL) any[tid] = 0;
+        if (tid < NL) {
+            any[tid] = 0;
+            if (MODE == 2 && FLAT) {
+                const int z = (int)fdiv(row0 + tid, p.d_l1);
+                at[tid] = z << 16 | (row0 + tid - z * p.L1);
+            }
+        }
         if (tid < 3) count[tid] = 0;
         __syncthreads();
         // ---- stage
@@ -286,6 +305,27 @@ __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__res
                 }
             }
             if (have) any[line] = 1;
+        } else if (FLAT) {
+            // the tile's lines are adjacent rows: flat positions, 4 loads in flight
+            for (int e0 = tid; e0 < nlines * L; e0 += 4 * T) {
+                int32_t f[4];
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    f[r] = -1;
+                    if (e0 + r * T < nlines * L)
+                        f[r] = MODE == 2 ? reinterpret_cast<const int32_t *>(src)[base + (e0 + r * T)]
+                                         : (int32_t) reinterpret_cast<const int16_t *>(src)[base + (e0 + r * T)];
+                }
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const int e = e0 + r * T;
+                    if (e >= nlines * L) break;
+                    const int l = (int)fdiv(e, p.d_line);
+                    const uint32_t v = MODE == 2 ? value01(f[r], at[l] >> 16, at[l] & 0xffff) : value0(f[r], row0 + l);
+                    g[e + l * (tl.pitch - L) + kLineK3] = v;
+                    if (v < kBig) any[l] = 1;
+                }
+            }
         } else {
             // units of 128 positions of a line, one warp each
             const int segs = (L + 127) / 128;
@@ -354,6 +394,7 @@ __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__res
             at = __shfl_sync(active, at, leader);
             if (wanted) list[which * NL * tl.blocks + at + __popc(want & ((1u << lane) - 1u))] = (uint16_t)task;
         };
+        bool wider = line < nlines && !any[line];
         for (int qb = slot; qb < tl.blocks; qb += kSlots) {
             const int q0 = qb * kLineQ;
             uint32_t key[kLineQ];
@@ -362,106 +403,112 @@ __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__res
             line_ring<-1, kLineK1>(gl + q0, cw, key);
             const uint32_t most = worst(key, q0);
             store(key, pl, q0);
-            append(0, live && most >= exact(kLineK1), line << kTaskBits | qb);
+            const bool wanted = live && most >= exact(kLineK1);
+            wider |= wanted;
+            append(0, wanted, line << kTaskBits | qb);
         }
-        __syncthreads();
-        for (int t = tid; t < count[0]; t += T) {
-            const int task = list[t], l = task >> kTaskBits, q0 = (task & kTaskMask) * kLineQ;
-            uint32_t key[kLineQ];
+        // (most tiles of a dense background end here, every value below the window's bound)
+        wider = __syncthreads_or(wider);
+        if (wider) {
+            for (int t = tid; t < count[0]; t += T) {
+                const int task = list[t], l = task >> kTaskBits, q0 = (task & kTaskMask) * kLineQ;
+                uint32_t key[kLineQ];
 #pragma unroll
-            for (int i = 0; i < kLineQ; i++) key[i] = 0xffffffffu;
-            line_ring<-1, kLineK2>(g + l * tl.pitch + kLineK3 + q0, cw, key);
-            const bool ok = worst(key, q0) < exact(kLineK2);
-            if (ok) store(key, pos + l * tl.ppitch, q0);
-            append(1, !ok, task);
-        }
-        __syncthreads();
-        // the positions the widest window leaves open: one by one from here on (list 0 again)
-        bool open = false;
-        for (int t = tid; t < count[1]; t += T) {
-            const int task = list[NL * tl.blocks + t], l = task >> kTaskBits, q0 = (task & kTaskMask) * kLineQ;
-            const uint32_t *gt = g + l * tl.pitch + kLineK3;
-            uint16_t *pt = pos + l * tl.ppitch;
-            uint32_t key[kLineQ];
-#pragma unroll
-            for (int i = 0; i < kLineQ; i++) key[i] = 0xffffffffu;
-            line_ring<-1, kLineK3>(gt + q0, cw, key);
-            if (worst(key, q0) < exact(kLineK3)) {
-                store(key, pt, q0);
-                continue;
-            }
-#pragma unroll
-            for (int i = 0; i < kLineQ; i++) {
-                if (q0 + i >= L) continue;
-                const int bp = min(max(q0 - kLineK3 + (int)(key[i] & 63u), 0), L - 1);  // (may point at padding)
-                bool done = key[i] < exact(kLineK3);
-                if (!done) {
-                    const uint32_t bound = gt[bp] + weight * (uint32_t)((q0 + i - bp) * (q0 + i - bp));
-                    const int at = bound < far_limit ? atomicAdd(&count[2], 1) : NL * tl.blocks;
-                    if (at < NL * tl.blocks) list[at] = (uint16_t)(l << kPosBits | (q0 + i));
-                    else open = true;
-                }
-                pt[q0 + i] = (uint16_t)(bp | (done ? 0 : kLineOpen));
-            }
-        }
-        __syncthreads();
-        for (int t = tid; t < min(count[2], NL * tl.blocks); t += T) {
-            const int l = list[t] >> kPosBits, q = list[t] & kPosMask;
-            const uint32_t *gt = g + l * tl.pitch + kLineK3 + q;
-            uint16_t *pt = pos + l * tl.ppitch + q;
-            int b = (*pt & (kLineOpen - 1)) - q;
-            uint32_t best = gt[b] + weight * (uint32_t)(b * b);
-            for (int k = kLineK3 + 1; weight * (uint32_t)(k * k) <= best; k++) {
-                const uint32_t d = weight * (uint32_t)(k * k);
-                const uint32_t left = q - k >= 0 ? gt[-k] + d : kBig;
-                const uint32_t right = q + k < L ? gt[k] + d : kBig;
-                if (left <= best) {  // equal: the lower position
-                    best = left;
-                    b = -k;
-                }
-                if (right < best) {
-                    best = right;
-                    b = k;
-                }
-            }
-            *pt = (uint16_t)(q + b);
-        }
-        // ---- halving, where a window left a position open
-        if (__syncthreads_or(open)) {
-            auto search = [&](int q, int lo, int hi) {
-                const int b = pl[q] & (kLineOpen - 1);
-                const uint32_t v0 = gl[b] + weight * (uint32_t)((q - b) * (q - b));
-                if (v0 < kBig) {  // nothing further than this can be better
-                    const int r = (int)sqrtf((float)v0 * inv_weight) + 1;
-                    lo = max(lo, q - r);
-                    hi = min(hi, q + r);
-                }
-                uint32_t best = 0xffffffffu;
-                int bp = lo;
-#pragma unroll 4
-                for (int pp = lo; pp <= hi; pp++) {
-                    const uint32_t v = gl[pp] + weight * (uint32_t)((q - pp) * (q - pp));
-                    if (v < best) {
-                        best = v;
-                        bp = pp;
-                    }
-                }
-                pl[q] = (uint16_t)bp;
-            };
-            int s = 1;
-            while (8 * s <= L) s *= 2;
-            if (live)
-                for (int q = slot * s; q < L; q += kSlots * s)
-                    if (pl[q] & kLineOpen) search(q, 0, L - 1);
-            for (s >>= 1; s > 0; s >>= 1) {
-                __syncthreads();
-                if (live)
-                    for (int q = s + 2 * s * slot; q < L; q += 2 * s * kSlots)
-                        if (pl[q] & kLineOpen) search(q, pl[q - s], q + s < L ? pl[q + s] : L - 1);
+                for (int i = 0; i < kLineQ; i++) key[i] = 0xffffffffu;
+                line_ring<-1, kLineK2>(g + l * tl.pitch + kLineK3 + q0, cw, key);
+                const bool ok = worst(key, q0) < exact(kLineK2);
+                if (ok) store(key, pos + l * tl.ppitch, q0);
+                append(1, !ok, task);
             }
             __syncthreads();
+            // the positions the widest window leaves open: one by one from here on (list 0 again)
+            bool open = false;
+            for (int t = tid; t < count[1]; t += T) {
+                const int task = list[NL * tl.blocks + t], l = task >> kTaskBits, q0 = (task & kTaskMask) * kLineQ;
+                const uint32_t *gt = g + l * tl.pitch + kLineK3;
+                uint16_t *pt = pos + l * tl.ppitch;
+                uint32_t key[kLineQ];
+#pragma unroll
+                for (int i = 0; i < kLineQ; i++) key[i] = 0xffffffffu;
+                line_ring<-1, kLineK3>(gt + q0, cw, key);
+                if (worst(key, q0) < exact(kLineK3)) {
+                    store(key, pt, q0);
+                    continue;
+                }
+#pragma unroll
+                for (int i = 0; i < kLineQ; i++) {
+                    if (q0 + i >= L) continue;
+                    const int bp = min(max(q0 - kLineK3 + (int)(key[i] & 63u), 0), L - 1);  // (may point at padding)
+                    bool done = key[i] < exact(kLineK3);
+                    if (!done) {
+                        const uint32_t bound = gt[bp] + weight * (uint32_t)((q0 + i - bp) * (q0 + i - bp));
+                        const int at = bound < far_limit ? atomicAdd(&count[2], 1) : NL * tl.blocks;
+                        if (at < NL * tl.blocks) list[at] = (uint16_t)(l << kPosBits | (q0 + i));
+                        else open = true;
+                    }
+                    pt[q0 + i] = (uint16_t)(bp | (done ? 0 : kLineOpen));
+                }
+            }
+            __syncthreads();
+            for (int t = tid; t < min(count[2], NL * tl.blocks); t += T) {
+                const int l = list[t] >> kPosBits, q = list[t] & kPosMask;
+                const uint32_t *gt = g + l * tl.pitch + kLineK3 + q;
+                uint16_t *pt = pos + l * tl.ppitch + q;
+                int b = (*pt & (kLineOpen - 1)) - q;
+                uint32_t best = gt[b] + weight * (uint32_t)(b * b);
+                for (int k = kLineK3 + 1; weight * (uint32_t)(k * k) <= best; k++) {
+                    const uint32_t d = weight * (uint32_t)(k * k);
+                    const uint32_t left = q - k >= 0 ? gt[-k] + d : kBig;
+                    const uint32_t right = q + k < L ? gt[k] + d : kBig;
+                    if (left <= best) {  // equal: the lower position
+                        best = left;
+                        b = -k;
+                    }
+                    if (right < best) {
+                        best = right;
+                        b = k;
+                    }
+                }
+                *pt = (uint16_t)(q + b);
+            }
+            // ---- halving, where a window left a position open
+            if (__syncthreads_or(open)) {
+                auto search = [&](int q, int lo, int hi) {
+                    const int b = pl[q] & (kLineOpen - 1);
+                    const uint32_t v0 = gl[b] + weight * (uint32_t)((q - b) * (q - b));
+                    if (v0 < kBig) {  // nothing further than this can be better
+                        const int r = (int)sqrtf((float)v0 * inv_weight) + 1;
+                        lo = max(lo, q - r);
+                        hi = min(hi, q + r);
+                    }
+                    uint32_t best = 0xffffffffu;
+                    int bp = lo;
+#pragma unroll 4
+                    for (int pp = lo; pp <= hi; pp++) {
+                        const uint32_t v = gl[pp] + weight * (uint32_t)((q - pp) * (q - pp));
+                        if (v < best) {
+                            best = v;
+                            bp = pp;
+                        }
+                    }
+                    pl[q] = (uint16_t)bp;
+                };
+                int s = 1;
+                while (8 * s <= L) s *= 2;
+                if (live)
+                    for (int q = slot * s; q < L; q += kSlots * s)
+                        if (pl[q] & kLineOpen) search(q, 0, L - 1);
+                for (s >>= 1; s > 0; s >>= 1) {
+                    __syncthreads();
+                    if (live)
+                        for (int q = s + 2 * s * slot; q < L; q += 2 * s * kSlots)
+                            if (pl[q] & kLineOpen) search(q, pl[q - s], q + s < L ? pl[q + s] : L - 1);
+                }
+                __syncthreads();
+            }
         }
         // ---- outputs
+        const bool near = !wider && weight * ((kLineK1 + 1) * (kLineK1 + 1)) <= kSqrtTab;  // root holds every value
         if (MODE == 1) {
             if (line < nlines) {
                 const bool site = any[line] != 0;
@@ -474,6 +521,70 @@ __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__res
                             (b << 16);
                     }
                     c2[o] = f;
+                }
+            }
+        } else if (FLAT) {
+            for (int e0 = tid; e0 < nlines * L; e0 += 4 * T) {
+                int l[4], b[4];
+                uint32_t v[4];
+                bool site[4];
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const int e = min(e0 + r * T, nlines * L - 1);
+                    l[r] = (int)fdiv(e, p.d_line);
+                    b[r] = pos[e + l[r] * (tl.ppitch - L)];
+                    site[r] = any[l[r]] != 0;
+                    if (!site[r]) b[r] = 0;
+                }
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const int q = min(e0 + r * T, nlines * L - 1) - l[r] * L, d = q - b[r];
+                    v[r] = g[l[r] * tl.pitch + kLineK3 + b[r]] + weight * (uint32_t)(d * d);
+                    if (!site[r]) {  // no background in the item: the site (-1, 0, ...)
+                        const int z = MODE == 2 ? at[l[r]] >> 16 : 0, y = MODE == 2 ? at[l[r]] & 0xffff : row0 + l[r];
+                        v[r] = w0 * (uint32_t)(MODE == 2 ? (z + 1) * (z + 1) : (y + 1) * (y + 1)) +
+                               (MODE == 2 ? w1 * (uint32_t)(y * y) : 0u) + weight * (uint32_t)(q * q);
+                    }
+                }
+                if (dist) {
+                    float d[4];
+                    if (near) {
+#pragma unroll
+                        for (int r = 0; r < 4; r++) d[r] = root[min(v[r], kSqrtTab - 1u)];  // (beyond the line: any entry)
+                    } else {
+#pragma unroll
+                        for (int r = 0; r < 4; r++) d[r] = line_dist(v[r], p.unit2);
+                    }
+#pragma unroll
+                    for (int r = 0; r < 4; r++)
+                        if (e0 + r * T < nlines * L) __stcs(dist + base + (e0 + r * T), d[r]);
+                }
+                if (OUT == 0) continue;  // distances only
+                if (sqdist) {
+#pragma unroll
+                    for (int r = 0; r < 4; r++)
+                        if (e0 + r * T < nlines * L) __stcs(sqdist + base + (e0 + r * T), (int32_t)v[r]);
+                }
+                if (indices) {
+                    int32_t f[4];
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const int64_t o = base + l[r] * L + b[r];
+                        f[r] = MODE == 2 ? reinterpret_cast<const int32_t *>(src)[o]
+                                         : (int32_t) reinterpret_cast<const int16_t *>(src)[o];
+                    }
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        if (e0 + r * T >= nlines * L) continue;
+                        int32_t *o = indices + base + (e0 + r * T);
+                        __stcs(o, site[r] ? (MODE == 2 ? (int32_t)(int16_t)(f[r] & 0xffff) : f[r]) : -1);
+                        if (MODE == 2) {
+                            __stcs(o + p.numel, site[r] ? f[r] >> 16 : 0);
+                            __stcs(o + 2 * p.numel, b[r]);
+                        } else {
+                            __stcs(o + p.numel, b[r]);
+                        }
+                    }
                 }
             }
         } else {
@@ -506,11 +617,17 @@ __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__res
                     }
                 }
                 if (dist) {
+                    float d[4];
+                    if (near) {
 #pragma unroll
-                    for (int r = 0; r < 4; r++) {
-                        const float d = line_dist(v[r], p.unit2);
-                        if (q0 + 32 * r < L) __stcs(dist + gi + 32 * r, d);
+                        for (int r = 0; r < 4; r++) d[r] = root[min(v[r], kSqrtTab - 1u)];  // (beyond the line: any entry)
+                    } else {
+#pragma unroll
+                        for (int r = 0; r < 4; r++) d[r] = line_dist(v[r], p.unit2);
                     }
+#pragma unroll
+                    for (int r = 0; r < 4; r++)
+                        if (q0 + 32 * r < L) __stcs(dist + gi + 32 * r, d[r]);
                 }
                 if (OUT == 0) continue;  // distances only
                 if (sqdist) {
