@@ -282,6 +282,7 @@ __global__ void __launch_bounds__(kBThreads) bitmorph_kernel(const uint8_t *__re
 // HW .. 31 - HW write their word as 32 bytes (two 16-byte stores).
 constexpr int kWalkBRows = 32;   // output rows per task
 constexpr int kWalkBChunk = 4;   // input rows whose loads are in flight together
+constexpr int64_t kWalkBMinWords = 1200000;  // smaller batches run on tiles
 
 struct BitRows {  // an operator's taps grouped by row offset dy = k - hy
     int n[5];
@@ -476,6 +477,12 @@ int try_walk(const BitOps &ops, const uint8_t *in, uint8_t *out, int64_t batch, 
     const int sw = 32 - 2 * (fused ? 2 : 1);
     a.strips = (int)ceil_div(a.nw, sw);
     a.rblocks = (int)ceil_div(H, kWalkBRows);
+    // A strip is a serial chain of rows (3 us a tap at any size): the walkers pay once there are
+    // strips for every SM, most of their lanes with a word of the item.  Erosion, tiles against
+    // walkers: 3 x 3 of 8 x 4096^2 117 and 68 us, of 8 x 2048^2 29 and 38, of 64 x 128^2 3.8 and
+    // 34; cross of 10 x 2048^2 33 and 29, of 2000 x 256^2 106 and 127; 5 x 5 of 64 x 128^2 4.5 and 68.
+    const int64_t words = batch * H * a.nw;
+    if (words < kWalkBMinWords || 5 * a.nw < 3 * 32 * a.strips) return TM_OK;
     int st;
     if (!fused)
         st = hy == 0 ? launch_walk<0, 0, false>(in, out, a, s)

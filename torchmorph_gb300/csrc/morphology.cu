@@ -31,7 +31,7 @@
 namespace tmc {
 namespace {
 
-constexpr size_t kBitBoxTaps = 25;  // binary boxes of more voxels run on byte tiles
+constexpr size_t kBitBoxTaps = 65;  // binary boxes of more voxels run on byte tiles
 
 using namespace morph;
 
@@ -429,7 +429,8 @@ int run_morphology(const T *in, T *out, int64_t batch, int ndim, const int64_t *
     if constexpr (sizeof(T) == 1) {
         // binary, 1-D / 2-D: bit-packed tiles, except for larger full boxes, which the
         // separable byte tiles take (a tap costs an operation per word, a box's window
-        // two per row and column: 3 x 3 on 8 x 4096^2 73 us in bits, 208 us in bytes)
+        // two per row and column).  4 x 2048^2, bits and bytes: 3 x 3 16 and 38 us, 5 x 5 21 and 39,
+        // 33 x 1 24 and 50, 8 x 8 33 and 38, 1 x 65 32 and 85, 9 x 9 39 and 39, 11 x 11 52 and 44
         if (ndim <= 2 && !(box && taps.size() > kBitBoxTaps)) {
             bool done = false;
             st = bitmorph_uniform(MAX ? 1 : 0, in, out, batch, ndim, shape, footprint, sshape, origin, cval != 0.0f,
