@@ -86,25 +86,35 @@ constexpr int kTileW = 128;
 constexpr int kTileH = 32;
 constexpr int kFlatThreads = 256;
 constexpr int kRun = 8;
-// Row pitch of the row-pass buffer: odd, so that threads writing the same
-// column of consecutive rows hit different banks.
-constexpr int kRowsPitch = kTileW + 1;
+// Row pitches, in elements, of the row-pass buffer and of a staged tile for a window of kw
+// columns (room for full runs past the last column).  An odd number of 4-byte words: threads
+// on the same column of consecutive rows then hit different banks, of bytes as of floats
+// (binary 45 x 45 of 4 x 2048^2 160 us with an odd number of bytes, 1 x 66 86 us).
+template <typename T>
+constexpr int kRowsPitch = sizeof(T) == 4 ? kTileW + 1 : kTileW + 4;
+template <typename T>
+__host__ __device__ inline int stage_pitch(int kw) {
+    constexpr int per_word = 4 / (int)sizeof(T);
+    return (((kTileW + kw - 1 + (kRun - 1) + per_word - 1) / per_word) | 1) * per_word;
+}
 
-// Row pitch of a staged tile for a window of kw columns: room for full runs
-// past the last column, made odd so that consecutive rows start in different
-// banks (the row pass gives consecutive rows to consecutive threads).
-__host__ __device__ inline int stage_pitch(int kw) { return (kTileW + kw - 1 + (kRun - 1)) | 1; }
+// Shared memory of a tile for a window of runtime size: the staged tile and, for windows of more
+// than one column, the row pass.
+template <typename T>
+inline size_t flat_smem(int kh, int kw) {
+    return (size_t)(kTileH + kh - 1) * (stage_pitch<T>(kw) + (kw > 1 ? kRowsPitch<T> : 0)) * sizeof(T);
+}
 
 // Stage rows [gy0, gy0 + RH) x columns [gx0, gx0 + RW) of one H x W image into shared
 // memory (row stride ld), mapping out-of-image coordinates with the border mode.  Warp w
-// takes rows w, w + 8, ...; a lane maps its up to 5 columns of a chunk once for all rows
+// takes rows w, w + 8, ...; a lane maps its NC columns of a chunk once for all rows
 // and issues the loads of 2 rows before it stores any, so border tiles cost what
-// interior ones do and a warp keeps 10 loads in flight.
-template <typename T>
-__device__ __forceinline__ void stage_tile(const T *__restrict__ src, int H, int W, int gy0, int gx0, int RH, int RW,
-                                           int ld, int mode, T cval, T *tile) {
+// interior ones do and a warp keeps 2 NC loads in flight.
+template <typename T, int NC>
+__device__ __forceinline__ void stage_columns(const T *__restrict__ src, int H, int W, int gy0, int gx0, int RH,
+                                              int RW, int ld, int mode, T cval, T *tile) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int nwarps = kFlatThreads / 32, RB = 2, NC = 5;
+    constexpr int nwarps = kFlatThreads / 32, RB = 2;
     for (int cb = lane; cb < RW; cb += 32 * NC) {
         int mx[NC];  // -1: the constant; columns past the region repeat one inside it, unstored
 #pragma unroll
@@ -130,6 +140,14 @@ __device__ __forceinline__ void stage_tile(const T *__restrict__ src, int H, int
             }
         }
     }
+}
+
+template <typename T>
+__device__ __forceinline__ void stage_tile(const T *__restrict__ src, int H, int W, int gy0, int gx0, int RH, int RW,
+                                           int ld, int mode, T cval, T *tile) {
+    // (one chunk up to 192 columns: binary 9 x 45 of 4 x 2048^2 62 us with two)
+    if (RW > 160 && RW <= 192) stage_columns<T, 6>(src, H, W, gy0, gx0, RH, RW, ld, mode, cval, tile);
+    else stage_columns<T, 5>(src, H, W, gy0, gx0, RH, RW, ld, mode, cval, tile);
 }
 
 struct Flat2DParams {
@@ -187,7 +205,7 @@ __device__ __forceinline__ void window_run(const T *src, int step, int k, T *res
 }
 
 // Row pass then column pass of one staged tile: `tile` points at the first
-// input column the tile needs (odd row stride ld), `rows` receives the row-pass
+// input column the tile needs (row stride ld), `rows` receives the row-pass
 // result (RH x kTileW at pitch kRowsPitch); outputs go to dst at (y0.., x0..).
 // (RH rows of the region and the columns inside the item are computed; d_rows divides by RH.)
 template <typename T, bool MAX>
@@ -198,30 +216,37 @@ __device__ __forceinline__ void flat_tile_compute(const T *tile, int ld, T *rows
     const int runs = (cols + kRun - 1) / kRun;
     // (every row of the region, also below the outputs of a tile at the item's end: the
     // work unit's division stays a constant one; those rows are stale and unused)
+    constexpr int kPitch = kRowsPitch<T>;
+    auto column_pass = [&](const T *from, int pitch) {
+        for (int w = threadIdx.x; w < kTileW * (kTileH / kRun); w += kFlatThreads) {
+            const int c = w % kTileW, r = (w / kTileW) * kRun;
+            if (c >= cols || r >= outs) continue;
+            // kTileH is a multiple of kRun, so the run reads rows
+            // r .. r + kRun + kh - 2 <= RH - 1: always inside the row buffer
+            T res[kRun];
+            window_run<T, MAX>(from + r * pitch + c, pitch, p.kh, res);
+            T *o = dst + (int64_t)(y0 + r) * p.W + x0 + c;
+#pragma unroll
+            for (int j = 0; j < kRun; j++, o += p.W)
+                if (r + j < outs) __stcs(o, MorphOp<T, MAX>::apply(res[j], p.sval));
+        }
+    };
+    if (p.kw == 1) {  // no row pass (and no buffer for one: 81 x 1 of 4 x 2048^2 207 us with it)
+        column_pass(tile, ld);
+        return;
+    }
     for (int w = threadIdx.x; w < RH * runs; w += kFlatThreads) {
-        // consecutive threads take the same run of consecutive rows (odd row stride)
+        // consecutive threads take the same run of consecutive rows
         const int u = (int)fdiv(w, p.d_rows), r = w - u * RH;
         if (r >= outs + p.kh - 1) continue;
         const int c = kRun * u;
         T res[kRun];
         window_run<T, MAX>(tile + r * ld + c, 1, p.kw, res);
 #pragma unroll
-        for (int j = 0; j < kRun; j++) rows[r * kRowsPitch + c + j] = res[j];
+        for (int j = 0; j < kRun; j++) rows[r * kPitch + c + j] = res[j];
     }
     __syncthreads();
-    const int runs_per_col = kTileH / kRun;
-    for (int w = threadIdx.x; w < kTileW * runs_per_col; w += kFlatThreads) {
-        const int c = w % kTileW, r = (w / kTileW) * kRun;
-        if (c >= cols || r >= outs) continue;
-        // kTileH is a multiple of kRun, so the run reads rows
-        // r .. r + kRun + kh - 2 <= RH - 1: always inside the row buffer
-        T res[kRun];
-        window_run<T, MAX>(rows + r * kRowsPitch + c, kRowsPitch, p.kh, res);
-        T *o = dst + (int64_t)(y0 + r) * p.W + x0 + c;
-#pragma unroll
-        for (int j = 0; j < kRun; j++, o += p.W)
-            if (r + j < outs) __stcs(o, MorphOp<T, MAX>::apply(res[j], p.sval));
-    }
+    column_pass(rows, kPitch);
 }
 
 // Compile-time window (KH x KW): each thread walks down one column of the

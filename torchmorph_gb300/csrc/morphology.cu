@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kFlatThreads) flat2d_kernel(const T *__restric
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int RH = kTileH + p.kh - 1;      // loaded rows
     const int RW = kTileW + p.kw - 1;      // loaded columns
-    const int RWp = stage_pitch(p.kw);     // padded so full runs never read past a row; odd
+    const int RWp = stage_pitch<T>(p.kw);
     T *tile = reinterpret_cast<T *>(smem_raw);
     T *rows = tile + RH * RWp;             // row-pass result, RH x kTileW at pitch kRowsPitch
     const int x0 = blockIdx.x * kTileW;
@@ -360,9 +360,8 @@ int launch_flat2d_small(const T *in, T *out, Flat2DParams p, int64_t batch, int 
 // Flat 1-D/2-D box, a CTA per tile or persistent TMA-staged tiles.
 template <typename T, bool MAX, int KH, int KW>
 int launch_flat2d(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, cudaStream_t stream) {
-    const int RH = kTileH + p.kh - 1, RWp = stage_pitch(p.kw);
-    const size_t rows_bytes = KH == 0 ? (size_t)RH * kRowsPitch * sizeof(T) : 0;
-    const size_t smem = (size_t)RH * RWp * sizeof(T) + rows_bytes;
+    const int RH = kTileH + p.kh - 1;
+    const size_t smem = KH == 0 ? flat_smem<T>(p.kh, p.kw) : (size_t)RH * stage_pitch<T>(p.kw) * sizeof(T);
     const int st = allow_shared_memory((const void *)flat2d_kernel<T, MAX, KH, KW>, smem);
     if (st != TM_OK) return st;
     dim3 grid((unsigned)ceil_div(p.W, kTileW), (unsigned)ceil_div(p.H, kTileH),
@@ -465,8 +464,7 @@ int run_morphology(const T *in, T *out, int64_t batch, int ndim, const int64_t *
         p.d_rows = make_fastdiv(kTileH + p.kh - 1);
         if (p.kh > 4096 || p.kw > 4096) goto stencil;  // tile would not fit on chip
         {
-            const int RH = kTileH + p.kh - 1, RW = stage_pitch(p.kw);
-            if ((size_t)RH * RW * sizeof(T) + (size_t)RH * kRowsPitch * sizeof(T) > 200 * 1024) goto stencil;
+            if (flat_smem<T>(p.kh, p.kw) > 200 * 1024) goto stencil;
             if constexpr (sizeof(T) == 4) {
                 // centred 3 x 3 / 5 x 5 windows on 16-byte aligned rows: register
                 // walkers for the interior, one thread per output for the frame

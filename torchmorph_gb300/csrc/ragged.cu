@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kFlatThreads) ragged_flat_kernel(const T *__re
     __shared__ int s_slot[2];
     __shared__ int s_tb[kQueueCache];
     const int RH = kTileH + w.kh - 1, RW = kTileW + w.kw - 1;
-    const int RWp = stage_pitch(w.kw);
+    const int RWp = stage_pitch<T>(w.kw);
     T *tile = reinterpret_cast<T *>(smem_raw);
     T *rows = tile + RH * RWp;
     TileQueue<RaggedItem> q{&hdr->queue, hdr->ntiles, hdr->nitems, items, s_tb, s_slot, 0};
@@ -211,8 +211,8 @@ int persistent_grid(K kernel, size_t smem, int *grid) {
 template <typename T, bool MAX, int KH, int KW>
 int launch_ragged_flat(const T *in, T *out, PlanHeader *hdr, const RaggedItem *items, const RaggedWindow &w,
                        cudaStream_t s) {
-    const int RH = kTileH + w.kh - 1, RWp = stage_pitch(w.kw);
-    const size_t smem = (size_t)RH * RWp * sizeof(T) + (KH == 0 ? (size_t)RH * kRowsPitch * sizeof(T) : 0);
+    const size_t smem =
+        (size_t)(kTileH + w.kh - 1) * (stage_pitch<T>(w.kw) + (KH == 0 ? kRowsPitch<T> : 0)) * sizeof(T);
     auto kernel = ragged_flat_kernel<T, MAX, KH, KW>;
     int grid = 0;
     int st = persistent_grid(kernel, smem, &grid);
