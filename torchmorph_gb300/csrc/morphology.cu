@@ -45,14 +45,17 @@ __global__ void __launch_bounds__(kFlatThreads) flat2d_kernel(const T *__restric
     T *tile = reinterpret_cast<T *>(smem_raw);
     T *rows = tile + RH * RWp;             // row-pass result, RH x kTileW at pitch kRowsPitch
     const int x0 = blockIdx.x * kTileW;
-    const int y0 = blockIdx.y * kTileH;
     for (int64_t item = blockIdx.z; item < p.batch; item += gridDim.z) {
         const int64_t off = item * (int64_t)p.H * p.W;
-        stage_tile<T>(in + off, p.H, p.W, y0 + p.lo_y, x0 + p.lo_x, min(RH, p.H - y0 + p.kh - 1),
-                      min(RW, p.W - x0 + p.kw - 1), RWp, p.mode, (T)p.cval, tile);
-        __syncthreads();
-        tile_compute<T, MAX, KH, KW>(tile, RWp, rows, p, out + off, x0, y0);
-        __syncthreads();
+        // (one turn but for items of more than 65535 rows of tiles, the most a grid has)
+        for (int64_t y1 = (int64_t)blockIdx.y * kTileH; y1 < p.H; y1 += (int64_t)gridDim.y * kTileH) {
+            const int y0 = (int)y1;
+            stage_tile<T>(in + off, p.H, p.W, y0 + p.lo_y, x0 + p.lo_x, min(RH, p.H - y0 + p.kh - 1),
+                          min(RW, p.W - x0 + p.kw - 1), RWp, p.mode, (T)p.cval, tile);
+            __syncthreads();
+            tile_compute<T, MAX, KH, KW>(tile, RWp, rows, p, out + off, x0, y0);
+            __syncthreads();
+        }
     }
 }
 
@@ -364,7 +367,7 @@ int launch_flat2d(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, c
     const size_t smem = KH == 0 ? flat_smem<T>(p.kh, p.kw) : (size_t)RH * stage_pitch<T>(p.kw) * sizeof(T);
     const int st = allow_shared_memory((const void *)flat2d_kernel<T, MAX, KH, KW>, smem);
     if (st != TM_OK) return st;
-    dim3 grid((unsigned)ceil_div(p.W, kTileW), (unsigned)ceil_div(p.H, kTileH),
+    dim3 grid((unsigned)ceil_div(p.W, kTileW), (unsigned)std::min<int64_t>(ceil_div(p.H, kTileH), 65535),
               (unsigned)(batch < 65535 ? batch : 65535));
     // windows of a runtime size: their row pass wants an odd row pitch, which a TMA box
     // cannot have (15 x 15 on 4 x 2048^2: 53 us, 98 us through TMA-staged tiles)
