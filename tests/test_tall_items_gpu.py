@@ -22,3 +22,13 @@ def test_tall_flat_windows(cuda, width):
             part = op(v[:, :, lo:hi].contiguous())
             a, b = (0 if lo == 0 else 10), (None if hi == ROWS else -10)
             assert torch.equal(whole[:, :, lo:hi][:, :, a:b], part[:, :, a:b])
+
+
+def test_tall_staged_tiles(cuda):
+    """The persistent kernel of compile-time windows (aligned rows of more than a tile)."""
+    x = torch.rand((1, 1, ROWS, 144), generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    whole = tm.grey_dilation(x, size=3, origin=1)
+    for lo, hi in ((0, 500), (65535 * 32 - 300, 65535 * 32 + 300), (ROWS - 500, ROWS)):
+        part = tm.grey_dilation(x[:, :, lo:hi].contiguous(), size=3, origin=1)
+        a, b = (0 if lo == 0 else 10), (None if hi == ROWS else -10)
+        assert torch.equal(whole[:, :, lo:hi][:, :, a:b], part[:, :, a:b])

@@ -297,7 +297,7 @@ int launch_flat2d_small(const T *in, T *out, Flat2DParams p, int64_t batch, int 
     tp.align = 16 / (int)sizeof(T);
     tp.bw = (int)round_up((size_t)(kTileW + p.kw - 1 + tp.align - 1), (size_t)tp.align);
     tp.ntx = (int)grid.x;
-    tp.nty = (int)grid.y;
+    tp.nty = (int)ceil_div(p.H, kTileH);  // (grid.y has a limit)
     tp.ntiles = (int64_t)tp.ntx * tp.nty * batch;
     {
         // interior tile rows/columns: the region of tile t starts at
