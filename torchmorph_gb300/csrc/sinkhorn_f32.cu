@@ -361,6 +361,7 @@ constexpr int kSlabRows = 8;       // rows per tile
 constexpr int kSlabMaxCtas = 160;  // CTAs of a launch (residual partials are sized for these)
 constexpr int kSlabWarps = kSkThreads / 32;
 constexpr int kSlabMaxGroups = 60;  // arrival counters in the control block
+constexpr int64_t kOneWaveMaxPairs = 1 << 14;  // larger batches are the tile kernel's by any of the rules below
 
 template <bool LOG, int V>
 struct SlabTile {
@@ -681,7 +682,7 @@ template <bool LOG, int V>
 inline bool slab_shape(int64_t n, int64_t d, int sms, SlabShape *out) {
     constexpr int PT = SlabTile<LOG, V>::PT, N = SlabTile<LOG, V>::N;
     const int64_t W = ceil_div(d, (int64_t)SlabTile<LOG, V>::kCols), sets = kSlabWarps / W;
-    if (W > kSlabWarps) return false;
+    if (W > kSlabWarps || n > kOneWaveMaxPairs) return false;
     int64_t best = 0;
     for (int rows = kSlabRows; rows <= 4 * kSlabRows; rows += kSlabRows) {
         SlabShape s;
@@ -1006,6 +1007,7 @@ int cluster_count(int ctas) {
 // stopping test they meet) the one with the least time, or false.  Any shape that fits beats
 // the slabs, whose half-steps never take less than 3.2 us.
 bool cluster_shape(int64_t n, int64_t d, ClusterShape *out) {
+    if (n > kOneWaveMaxPairs) return false;
     double best = 0;
     for (int ctas : {1, 2, 4, 6, 8, 10, 12, 16})
         for (int pairs = 1; pairs <= 4; pairs *= 2) {
@@ -1461,7 +1463,13 @@ struct SkLayout {
 SkLayout sk_layout(int64_t n, int64_t d, bool log_form, int64_t max_iter, int64_t check_every, bool line) {
     SkLayout L{};
     const size_t dd = (size_t)d * d * sizeof(float), nd = (size_t)n * d * sizeof(float);
-    const size_t rblocks = std::max((size_t)ceil_div(d, kSkRows), (size_t)kSlabMaxCtas);  // residual partials
+    // residual partials: a row per row block of the tile kernel, per CTA of a slab group, two per
+    // CTA of a cluster
+    size_t rblocks = (size_t)ceil_div(d, kSkRows);
+    if (n <= kOneWaveMaxPairs)
+        rblocks = std::max(rblocks, std::min((size_t)kSlabMaxCtas,
+                                             std::max((size_t)ceil_div(d, kSlabRows), (size_t)(2 * kClMaxCtas))));
+    if (check_every <= 0) rblocks = 0;
     const size_t checks = check_every > 0 ? (size_t)(max_iter / check_every) + 1 : 1;
     size_t off = 0;
     L.mat = off;
