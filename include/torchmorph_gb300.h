@@ -115,6 +115,10 @@ int tm_tune_variants(int op);
 int tm_tune_class(int op, int64_t a, int64_t b);
 int tm_tune_set(int op, int cls, int variant);
 int tm_tune_get(int op, int cls);
+/* How often the calling thread's operators have looked an `op` variant up so
+ * far: unchanged over a call that no variant applies to (a problem that another
+ * kernel takes).  -1 for an unknown op. */
+int64_t tm_tune_lookups(int op);
 
 /* ------------------------------------------------------------------ grey --
  * Replaces grey_erosion_cuda / grey_dilation_cuda

@@ -64,6 +64,7 @@ SIGNATURES = {
     "tm_tune_class": (c_int, [c_int, c_i64, c_i64]),
     "tm_tune_set": (c_int, [c_int, c_int, c_int]),
     "tm_tune_get": (c_int, [c_int, c_int]),
+    "tm_tune_lookups": (c_i64, [c_int]),
     "tm_sinkhorn_iter_workspace_size": (c_size, []),
     "tm_sinkhorn_fastiter": (c_int, [c_void, c_void, c_void, c_void, c_void, c_void, c_i64, c_i64,
                                      c_i64, c_void, c_size, c_void]),

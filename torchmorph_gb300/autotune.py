@@ -87,6 +87,11 @@ def variants(op: str) -> int:
     return int(_lib.load().tm_tune_variants(OPS[op]))
 
 
+def lookups(op: str) -> int:
+    """How often this thread's operators have looked an `op` variant up."""
+    return int(_lib.load().tm_tune_lookups(OPS[op]))
+
+
 def work_class(op: str, a: int, b: int = 0) -> int:
     return int(_lib.load().tm_tune_class(OPS[op], int(a), int(b)))
 
@@ -127,7 +132,12 @@ def tune(op: str, call: Callable[[], object], a: int, b: int = 0, *, warmup: int
     class is given by `a`, `b` as for :func:`work_class`), check that each returns the
     same bits as the built-in choice, keep the fastest for the class and, with
     `persist`, record it in the cache.  Returns {"class", "times_ms" (per variant),
-    "builtin_ms", "best"}."""
+    "builtin_ms", "best"}.
+
+    A call that another kernel takes whatever the variant (a Sinkhorn problem whose matrix
+    stays in shared memory, a box of the register walkers) tells nothing about its class:
+    the class keeps the choice that it had, `best` (-1: built-in), and the cache an entry
+    that it has; every variant's time is the call's."""
     if op not in OPS:
         raise ValueError(f"unknown operator {op!r}; one of {sorted(OPS)}")
     cls = work_class(op, a, b)
@@ -148,10 +158,12 @@ def tune(op: str, call: Callable[[], object], a: int, b: int = 0, *, warmup: int
 
     try:
         set_variant(op, cls, -1)
+        before = lookups(op)
         reference = _snapshot(call())
+        reached = lookups(op) != before
         builtin_ms = timed()
-        times = []
-        for v in range(variants(op)):
+        times = [] if reached else [builtin_ms] * variants(op)
+        for v in range(variants(op) if reached else 0):
             set_variant(op, cls, v)
             got = _snapshot(call())
             if len(got) != len(reference) or not all(torch.equal(x, y) for x, y in zip(got, reference)):
@@ -160,13 +172,15 @@ def tune(op: str, call: Callable[[], object], a: int, b: int = 0, *, warmup: int
     except Exception:
         set_variant(op, cls, previous)
         raise
-    best = min(range(len(times)), key=times.__getitem__)
+    best = min(range(len(times)), key=times.__getitem__) if reached else previous
     set_variant(op, cls, best)
     if persist:
         data = load_cache(path)
         name = torch.cuda.get_device_name(torch.cuda.current_device())
-        data["devices"].setdefault(name, {}).setdefault(op, {})[str(cls)] = best
-        save_cache(data, path)
+        table = data["devices"].setdefault(name, {}).setdefault(op, {})
+        if reached or str(cls) not in table:
+            table[str(cls)] = best  # (-1, the built-in choice, is skipped when a cache is applied)
+            save_cache(data, path)
     return {"class": cls, "times_ms": times, "builtin_ms": builtin_ms, "best": best}
 
 

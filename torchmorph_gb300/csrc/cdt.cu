@@ -448,9 +448,9 @@ extern "C" int tm_cdt(const void *input, int in_dtype, int64_t batch, int ndim, 
     bool cleared = false;
     // autotuned variants: 1 = the raster passes for every item (no shell search),
     // 2 = the shell search with one CTA per 32-row block instead of the warp queue
-    const int variant = tune_variant(kTuneCdt3D, tune_class(kTuneCdt3D, g.numel, 0));
-    const bool shell = variant != 1;
-    if (shell && cdt_shell_shape(g) && cdt_shell_eligible(g, dist, indices)) {
+    const bool fits = cdt_shell_shape(g) && cdt_shell_eligible(g, dist, indices);
+    const int variant = fits ? tune_variant(kTuneCdt3D, tune_class(kTuneCdt3D, g.numel, 0)) : -1;
+    if (fits && variant != 1) {
         // counters first, so that nothing but kernels follows the shell search
         TM_CHECK_CUDA(clear_cdt_counters(ws, pl, s));
         cleared = true;

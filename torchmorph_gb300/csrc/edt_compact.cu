@@ -1712,8 +1712,7 @@ int edt_compact_run(const void *input, int in_dtype, const Geometry &g, const Ed
     // multiples of 4 voxels here, so 2 bytes a voxel hold 4 per item).
     int *todo = nullptr;
     // autotuned variant 1: the separable passes for every item (no shell search)
-    const bool shell = tune_variant(kTuneEdt3D, tune_class(kTuneEdt3D, g.numel, 0)) != 1;
-    if (shell_shape && p.L2 <= 1024 && shell) {
+    if (shell_shape && p.L2 <= 1024 && tune_variant(kTuneEdt3D, tune_class(kTuneEdt3D, g.numel, 0)) != 1) {
         int st = TM_OK;
         const int ww = (p.L2 + 31) / 32;
         const int64_t nwords = g.batch * (int64_t)p.L0 * p.L1 * ww;

@@ -318,11 +318,12 @@ int launch_flat2d_small(const T *in, T *out, Flat2DParams p, int64_t batch, int 
     // batch has a few tiles per SM; otherwise the plain kernel does all
     // autotuned variant: 0 TMA-staged persistent tiles at full occupancy, 1 plain
     // loads (one CTA per tile), 2 / 3 TMA with at most 1 / 2 CTAs per SM
-    const int variant = tune_variant(kTuneGreyFlat2D, tune_class(kTuneGreyFlat2D, batch * (int64_t)p.H * p.W, 0));
-    const bool tma_ok = variant != 1 && (p.W % tp.align) == 0 && ((uintptr_t)in & 15) == 0 && tp.bw <= 256 &&
-                        RH <= 256 && p.H >= RH && p.W >= tp.bw && tp.ntiles >= 2LL * sms &&
-                        tp.ntiles < ((int64_t)1 << 31) && batch < ((int64_t)1 << 31);
-    if (!tma_ok) {
+    const bool tma_ok = (p.W % tp.align) == 0 && ((uintptr_t)in & 15) == 0 && tp.bw <= 256 && RH <= 256 &&
+                        p.H >= RH && p.W >= tp.bw && tp.ntiles >= 2LL * sms && tp.ntiles < ((int64_t)1 << 31) &&
+                        batch < ((int64_t)1 << 31);
+    const int variant =
+        tma_ok ? tune_variant(kTuneGreyFlat2D, tune_class(kTuneGreyFlat2D, batch * (int64_t)p.H * p.W, 0)) : -1;
+    if (!tma_ok || variant == 1) {
         flat2d_kernel<T, MAX, KH, KW><<<grid, kFlatThreads, smem, stream>>>(in, out, p);
         TM_LAUNCH_CHECK("flat2d_kernel");
         return TM_OK;

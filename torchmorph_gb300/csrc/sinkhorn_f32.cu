@@ -1431,10 +1431,10 @@ int sk_launch(bool log_form, SkArgs A, cudaStream_t s) {
     if (st != TM_OK) return st;
     A.status = status;
     A.spin_limit = grid_wait_budget();
-    // autotuned variant: bit 0 = 64 pairs per tile (else 16), bit 1 = one CTA per SM
-    // (else two); built-in: 64 pairs per tile above 24 pairs, two CTAs per SM
     if (sk_cluster(log_form, A, s, &st)) return st;
     if (sk_slab(log_form, A, s, &st)) return st;
+    // autotuned variant: bit 0 = 64 pairs per tile (else 16), bit 1 = one CTA per SM
+    // (else two); built-in: 64 pairs per tile above 24 pairs, two CTAs per SM
     const int variant = tune_variant(kTuneSinkhornF32, tune_class(kTuneSinkhornF32, A.n, A.d));
     const bool wide = variant < 0 ? A.n > 24 : (variant & 1) != 0;
     const void *kern;

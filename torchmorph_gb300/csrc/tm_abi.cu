@@ -181,10 +181,17 @@ int tune_class(int op, int64_t a, int64_t b) {
     return std::min(kTuneClasses - 1, floor_log2(std::max<int64_t>(a, 1)));
 }
 
-int tune_variant(int op, int cls) {
+static int table_variant(int op, int cls) {
     if (op < 0 || op >= kTuneOps || cls < 0 || cls >= kTuneClasses) return -1;
     tune_init();
     return g_tune[op][cls].load(std::memory_order_relaxed);
+}
+
+static thread_local int64_t g_tune_lookups[kTuneOps] = {};
+
+int tune_variant(int op, int cls) {
+    g_tune_lookups[op]++;
+    return table_variant(op, cls);
 }
 
 static std::atomic<long long> g_grid_wait_budget{kSpinLimit};
@@ -214,7 +221,11 @@ extern "C" int tm_tune_set(int op, int cls, int variant) {
     return TM_OK;
 }
 
-extern "C" int tm_tune_get(int op, int cls) { return tmc::tune_variant(op, cls); }
+extern "C" int tm_tune_get(int op, int cls) { return tmc::table_variant(op, cls); }
+
+extern "C" int64_t tm_tune_lookups(int op) {
+    return op < 0 || op >= tmc::kTuneOps ? -1 : tmc::g_tune_lookups[op];
+}
 
 extern "C" void tm_set_grid_wait_budget(int64_t polls) {
     tmc::g_grid_wait_budget.store(polls < 0 ? tmc::kSpinLimit : (long long)polls);

@@ -34,7 +34,8 @@ int allow_shared_memory(const void *kernel, size_t smem);
 
 // Implementation variants picked by the autotuner (tm_tune_set), per operator
 // and work class; -1 = the library's built-in choice.  Every variant of an
-// operator gives bit-identical results.
+// operator gives bit-identical results.  tune_variant() is asked only where the answer
+// matters: tm_tune_lookups() tells the autotuner whether a call reaches the variants.
 enum TuneOp { kTuneGreyFlat2D = 0, kTuneSinkhornF32 = 1, kTuneEdt3D = 2, kTuneCdt3D = 3, kTuneOps = 4 };
 int tune_variant(int op, int cls);
 int tune_class(int op, int64_t a, int64_t b);
