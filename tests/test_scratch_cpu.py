@@ -25,3 +25,5 @@ def test_sinkhorn_f32_scratch_holds_the_residuals_of_every_kernel():
     for n, d in [(1, 1), (16, 64), (16, 784), (300, 2048), (16384, 64), (3, 5000)]:
         rows = max(-(-d // 128), min(160, max(32, -(-d // 8))))
         assert size(n, d, 0, 100, 10, 0) - size(n, d, 0, 100, 0, 0) >= 8 * n * rows
+        rows = max(-(-d // 128), min(160, -(-d // 8)))  # (the log form has no clusters)
+        assert size(n, d, 1, 100, 10, 0) - size(n, d, 1, 100, 0, 0) >= 8 * n * rows
