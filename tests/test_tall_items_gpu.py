@@ -14,7 +14,8 @@ ROWS = 65535 * 32 + 3000
 def test_tall_flat_windows(cuda, width):
     x = torch.rand((1, 1, ROWS, width), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
     box = torch.ones((13, 7), dtype=torch.bool)  # (beyond the bit tiles)
-    for op, v in ((lambda t: tm.grey_dilation(t, size=7), x), (lambda t: tm.grey_erosion(t, size=(9, 1)), x),
+    for op, v in ((lambda t: tm.grey_dilation(t, size=7), x), (lambda t: tm.grey_dilation(t, size=(1, 3)), x),
+                  (lambda t: tm.grey_erosion(t, size=(9, 1)), x),
                   (lambda t: tm.binary_erosion(t, structure=box), x > 0.1)):
         whole = op(v)
         # rows on both sides of the last block's, and the end: as in a part of the item

@@ -45,17 +45,14 @@ __global__ void __launch_bounds__(kFlatThreads) flat2d_kernel(const T *__restric
     T *tile = reinterpret_cast<T *>(smem_raw);
     T *rows = tile + RH * RWp;             // row-pass result, RH x kTileW at pitch kRowsPitch
     const int x0 = blockIdx.x * kTileW;
+    const int y0 = (KH == 0 ? p.y_first : 0) + blockIdx.y * kTileH;
     for (int64_t item = blockIdx.z; item < p.batch; item += gridDim.z) {
         const int64_t off = item * (int64_t)p.H * p.W;
-        // (one turn but for items of more than 65535 rows of tiles, the most a grid has)
-        for (int64_t y1 = (int64_t)blockIdx.y * kTileH; y1 < p.H; y1 += (int64_t)gridDim.y * kTileH) {
-            const int y0 = (int)y1;
-            stage_tile<T>(in + off, p.H, p.W, y0 + p.lo_y, x0 + p.lo_x, min(RH, p.H - y0 + p.kh - 1),
-                          min(RW, p.W - x0 + p.kw - 1), RWp, p.mode, (T)p.cval, tile);
-            __syncthreads();
-            tile_compute<T, MAX, KH, KW>(tile, RWp, rows, p, out + off, x0, y0);
-            __syncthreads();
-        }
+        stage_tile<T>(in + off, p.H, p.W, y0 + p.lo_y, x0 + p.lo_x, min(RH, p.H - y0 + p.kh - 1),
+                      min(RW, p.W - x0 + p.kw - 1), RWp, p.mode, (T)p.cval, tile);
+        __syncthreads();
+        tile_compute<T, MAX, KH, KW>(tile, RWp, rows, p, out + off, x0, y0);
+        __syncthreads();
     }
 }
 
@@ -286,18 +283,41 @@ struct Tap {
     float val;
 };
 
+// One CTA per tile; items of more than 65535 rows of tiles, the most a grid has, in several
+// launches of the kernel for runtime sizes (a first row in the others' parameters, or a loop
+// over the rows, costs 4 to 10 % of 1 x 3 and 3 x 3 windows).
+template <typename T, bool MAX, int KH, int KW>
+int launch_flat2d_plain(const T *in, T *out, Flat2DParams p, cudaStream_t stream) {
+    constexpr int kMaxRows = 65535;
+    const int64_t rows = ceil_div(p.H, kTileH);
+    if constexpr (KH > 0) {
+        if (rows > kMaxRows) return launch_flat2d_plain<T, MAX, 0, 0>(in, out, p, stream);
+    }
+    const size_t smem =
+        KH == 0 ? flat_smem<T>(p.kh, p.kw) : (size_t)(kTileH + p.kh - 1) * stage_pitch<T>(p.kw) * sizeof(T);
+    const int st = allow_shared_memory((const void *)flat2d_kernel<T, MAX, KH, KW>, smem);
+    if (st != TM_OK) return st;
+    for (int64_t row = 0; row < rows; row += kMaxRows) {
+        p.y_first = (int)(row * kTileH);
+        const dim3 grid((unsigned)ceil_div(p.W, kTileW), (unsigned)std::min<int64_t>(rows - row, kMaxRows),
+                        (unsigned)std::min<int64_t>(p.batch, 65535));
+        flat2d_kernel<T, MAX, KH, KW><<<grid, kFlatThreads, smem, stream>>>(in, out, p);
+        TM_LAUNCH_CHECK("flat2d_kernel");
+    }
+    return TM_OK;
+}
+
 // Compile-time windows: persistent TMA-staged tiles once a batch has a few per SM and its
 // rows are 16-byte aligned (off-centre 3 x 3 on 8 x 4096^2: 205 us, 307 us with a CTA per
 // tile), else a CTA per tile.
 template <typename T, bool MAX, int KH, int KW>
-int launch_flat2d_small(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, dim3 grid, size_t smem,
-                        cudaStream_t stream) {
+int launch_flat2d_small(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, cudaStream_t stream) {
     const int RH = kTileH + p.kh - 1;
     TmaTileParams tp;
     tp.align = 16 / (int)sizeof(T);
     tp.bw = (int)round_up((size_t)(kTileW + p.kw - 1 + tp.align - 1), (size_t)tp.align);
-    tp.ntx = (int)grid.x;
-    tp.nty = (int)ceil_div(p.H, kTileH);  // (grid.y has a limit)
+    tp.ntx = (int)ceil_div(p.W, kTileW);
+    tp.nty = (int)ceil_div(p.H, kTileH);
     tp.ntiles = (int64_t)tp.ntx * tp.nty * batch;
     {
         // interior tile rows/columns: the region of tile t starts at
@@ -323,11 +343,7 @@ int launch_flat2d_small(const T *in, T *out, Flat2DParams p, int64_t batch, int 
                         batch < ((int64_t)1 << 31);
     const int variant =
         tma_ok ? tune_variant(kTuneGreyFlat2D, tune_class(kTuneGreyFlat2D, batch * (int64_t)p.H * p.W, 0)) : -1;
-    if (!tma_ok || variant == 1) {
-        flat2d_kernel<T, MAX, KH, KW><<<grid, kFlatThreads, smem, stream>>>(in, out, p);
-        TM_LAUNCH_CHECK("flat2d_kernel");
-        return TM_OK;
-    }
+    if (!tma_ok || variant == 1) return launch_flat2d_plain<T, MAX, KH, KW>(in, out, p, stream);
     CUtensorMap map;
     const uint64_t dims[3] = {(uint64_t)p.W, (uint64_t)p.H, (uint64_t)batch};
     const uint64_t strides[2] = {(uint64_t)p.W * sizeof(T), (uint64_t)p.W * p.H * sizeof(T)};
@@ -364,21 +380,10 @@ int launch_flat2d_small(const T *in, T *out, Flat2DParams p, int64_t batch, int 
 // Flat 1-D/2-D box, a CTA per tile or persistent TMA-staged tiles.
 template <typename T, bool MAX, int KH, int KW>
 int launch_flat2d(const T *in, T *out, Flat2DParams p, int64_t batch, int sms, cudaStream_t stream) {
-    const int RH = kTileH + p.kh - 1;
-    const size_t smem = KH == 0 ? flat_smem<T>(p.kh, p.kw) : (size_t)RH * stage_pitch<T>(p.kw) * sizeof(T);
-    const int st = allow_shared_memory((const void *)flat2d_kernel<T, MAX, KH, KW>, smem);
-    if (st != TM_OK) return st;
-    dim3 grid((unsigned)ceil_div(p.W, kTileW), (unsigned)std::min<int64_t>(ceil_div(p.H, kTileH), 65535),
-              (unsigned)(batch < 65535 ? batch : 65535));
     // windows of a runtime size: their row pass wants an odd row pitch, which a TMA box
     // cannot have (15 x 15 on 4 x 2048^2: 53 us, 98 us through TMA-staged tiles)
-    if constexpr (KH == 0) {
-        flat2d_kernel<T, MAX, KH, KW><<<grid, kFlatThreads, smem, stream>>>(in, out, p);
-        TM_LAUNCH_CHECK("flat2d_kernel");
-        return TM_OK;
-    } else {
-        return launch_flat2d_small<T, MAX, KH, KW>(in, out, p, batch, sms, grid, smem, stream);
-    }
+    if constexpr (KH == 0) return launch_flat2d_plain<T, MAX, KH, KW>(in, out, p, stream);
+    else return launch_flat2d_small<T, MAX, KH, KW>(in, out, p, batch, sms, stream);
 }
 
 template <typename T, bool MAX>
