@@ -34,7 +34,6 @@ namespace {
 
 constexpr uint32_t kBig = 1u << 26;  // "no site"; eligible shapes keep every real value below it
 constexpr int kKeyShift = 5;         // key = value << 5 | window position
-constexpr int kFar = 24;             // widest exact window before a line uses the envelope
 constexpr int kNear1 = 4;            // first window of pass 1: q-4 .. q+4
 constexpr int kNear2 = 2;            // first window of pass 2: q-2 .. q+2
 constexpr int kQB = 8;               // pass 1 outputs per register window
@@ -76,7 +75,7 @@ __device__ __forceinline__ uint32_t window_key(const uint32_t *w) {
 // exact radius isqrt(best).  G(p) reads the unshifted value for 0 <= p < L.
 // Returns false when the radius exceeds `far`.
 template <int K, typename GF>
-__device__ __forceinline__ bool widen(int q, int L, GF G, uint32_t &best, int &bp, int far = kFar) {
+__device__ __forceinline__ bool widen(int q, int L, GF G, uint32_t &best, int &bp, int far) {
     const int r = best >= kBig ? L : isqrt_floor(best);
     if (r > far) return false;
     const int lo = q - r < 0 ? 0 : q - r, hi = q + r >= L ? L - 1 : q + r;

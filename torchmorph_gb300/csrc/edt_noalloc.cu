@@ -59,9 +59,14 @@ extern "C" int tm_edt_noalloc(const void *input, int in_dtype, int64_t batch, in
     if (in_dtype != TM_F32 && in_dtype != TM_U8) return fail(TM_ERR_INVALID_ARGUMENT, "unknown input dtype %d", in_dtype);
     if (!dist && !indices && !sqdist) return fail(TM_ERR_INVALID_ARGUMENT, "at least one output must be requested");
     EdtSpacing spacing;
-    if (!edt_compact_eligible(g, nullptr, &spacing) || (g.ndim == 3 && g.shape[1] > 256))
+    if (!edt_compact_eligible(g, nullptr, &spacing))
         return fail(TM_ERR_UNSUPPORTED,
                     "tm_edt_noalloc handles 2-D or 3-D items with unit spacing only (use tm_edt with a workspace)");
+    if (g.ndim == 3 && g.shape[1] > 256)
+        return fail(TM_ERR_UNSUPPORTED,
+                    "tm_edt_noalloc handles 3-D items of at most 256 voxels along axis 1, got %lld (use tm_edt with a "
+                    "workspace)",
+                    (long long)g.shape[1]);
     const size_t need = edt_compact_workspace(g);
     if (need > kScratchBytes)
         return fail(TM_ERR_TOO_LARGE,
