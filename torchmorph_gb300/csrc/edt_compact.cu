@@ -1655,7 +1655,7 @@ int launch_bits0(const In *in, int16_t *c1, const CompactParams &p, const int *t
     // 4 columns per lane once they give every SM 8 warps (a warp per 32 rows and 128 columns):
     // 2 x 88 x 180 x 214 19 -> 11.5 us, 64 x 250 x 512 20 -> 14; at half as many 16 x 512^2 11 -> 14
     const bool wide = inner % 4 == 0 && ((uintptr_t)in & (4 * sizeof(In) - 1)) == 0 &&
-                      p.batch * (inner / 128) * nw >= (int64_t)sm_count() * 8;
+                      p.batch * (inner / 128) * wpc >= (int64_t)sm_count() * 8;
     const int cols = wide ? 128 : 32;
     const int groups = (int)std::max<int64_t>(1, std::min<int64_t>(kBitsWarps / wpc, ceil_div(inner, cols)));
     const int64_t blocks = p.batch * ceil_div(inner, (int64_t)cols * groups);
@@ -1771,18 +1771,21 @@ int edt_compact_run(const void *input, int in_dtype, const Geometry &g, const Ed
     // lines (68 KB at 1333 voxels) leave room for few CTAs
     auto rows = [&](auto mode, auto out, const void *src, int L) -> int {
         constexpr int M = decltype(mode)::value, O = decltype(out)::value;
-        // flat where units of 128 would idle for a third of their positions: rows of 130, 80, 63
-        // voxels gain 8, 4, 14 %, rows of 100 nothing, 202 lose 4 %
-        const bool flat = ceil_div(L, 128) * 128 * 2 > 3 * (int64_t)L;
-        // (whether tiles of n lines still give every SM a few)
-        auto fills = [&](int n) { return p.batch * ceil_div(M == 2 ? (int64_t)p.L0 * p.L1 : p.L0, n) >= 4 * (int64_t)sm_count(); };
+        // flat where units of 128 would idle for most of a line's last one: rows of 130 and 63 voxels
+        // gain 8 and 14 %; masks with rows of 157 .. 168 lose 4 to 7 %, rows of 202 4 %
+        const bool flat = ceil_div(L, 128) * 128 * 4 > 7 * (int64_t)L;
+        // (whether tiles of n lines give every SM k of them: 64 x 128^2 14.4 us in tiles of 32, 12.5 of
+        // 16; 64 x 251 x 76 masks 26.6 and 28.2)
+        auto fills = [&](int n, int k) {
+            return p.batch * ceil_div(M == 2 ? (int64_t)p.L0 * p.L1 : p.L0, n) >= k * (int64_t)sm_count();
+        };
         auto go = [&](auto lines) -> int {
             constexpr int NL = decltype(lines)::value;
             return flat ? launch_lines<M, NL, 256, O, true>(src, nullptr, dist, indices, sqdist, p, todo, stream)
                         : launch_lines<M, NL, 256, O, false>(src, nullptr, dist, indices, sqdist, p, todo, stream);
         };
-        if (L <= kShortLine && fills(32)) return go(std::integral_constant<int, 32>());
-        if (L <= kShortLine || (M == 2 && L <= 2 * kShortLine && fills(16))) return go(std::integral_constant<int, 16>());
+        if (L <= kShortLine && fills(32, 2)) return go(std::integral_constant<int, 32>());
+        if (L <= kShortLine || (M == 2 && L <= 2 * kShortLine && fills(16, 4))) return go(std::integral_constant<int, 16>());
         if (L <= kMediumLine) return go(std::integral_constant<int, 8>());
         return launch_lines<M, 8, 512, O>(src, nullptr, dist, indices, sqdist, p, todo, stream);
     };
