@@ -11,12 +11,15 @@ from torch import Tensor
 
 from .. import _C
 from .._validation import validate_bcs_input, validate_output
-from .structure import _host_constant, _normalize_origin, _offset_grid, _validate_origin
+from .structure import _HOST_CONSTANTS, _keep_host_constant, _normalize_origin, _offset_grid, _validate_origin
 
 
 def _default_structure(nd: int) -> Tensor:
     """The default element (cross, connectivity 1) on the CPU, built once per rank; read only."""
-    return _host_constant(("cross", nd), lambda: ((_offset_grid(nd, 1, "cpu") != 0).sum(dim=0) <= 1).contiguous())
+    cross = _HOST_CONSTANTS.get(nd)
+    if cross is None:
+        cross = _keep_host_constant(nd, ((_offset_grid(nd, 1, "cpu") != 0).sum(dim=0) <= 1).contiguous())
+    return cross
 
 
 def _normalize_structure(structure: Tensor | None, spatial_ndim: int, name: str = "structure"):

@@ -14,7 +14,7 @@ from torch import Tensor
 
 from .. import _C
 from .._validation import validate_bcs_input, validate_output
-from .structure import _host_constant, _normalize_origin, _validate_origin
+from .structure import _HOST_CONSTANTS, _keep_host_constant, _normalize_origin, _validate_origin
 
 _MODE_MAP = {
     "constant": 0,
@@ -38,9 +38,12 @@ def _host_zeros(size: tuple) -> Tensor:
 def _box(size) -> Tensor:
     """The flat box of a `size` argument; small ones are built once (read only)."""
     size = tuple(map(operator.index, size))
-    if math.prod(size) > 4096:
-        return _host_zeros(size)
-    return _host_constant(size, lambda: _host_zeros(size))
+    box = _HOST_CONSTANTS.get(size)
+    if box is None:
+        box = _host_zeros(size)
+        if math.prod(size) <= 4096:
+            _keep_host_constant(size, box)
+    return box
 
 
 _NO_FOOTPRINT = torch.empty(0, dtype=torch.bool, device="cpu")

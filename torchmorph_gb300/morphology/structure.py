@@ -11,18 +11,14 @@ def _offset_grid(rank: int, radius: int, device=None) -> Tensor:
     return torch.stack(torch.meshgrid(*axes, indexing="ij"), dim=0)
 
 
+# CPU tensors that nothing writes to, built once per key.  Only plain tensors with memory of their
+# own: one built under a fake-tensor or functional mode belongs to that mode.
 _HOST_CONSTANTS: dict = {}
 
 
-def _host_constant(key, make) -> Tensor:
-    """`make()`, a CPU tensor that nothing writes to, built once per `key`.  Kept only if it is a
-    plain tensor with memory of its own: one built under a fake-tensor or functional mode
-    belongs to that mode."""
-    t = _HOST_CONSTANTS.get(key)
-    if t is None:
-        t = make()
-        if type(t) is Tensor and t.data_ptr() != 0 and len(_HOST_CONSTANTS) < 256:
-            _HOST_CONSTANTS[key] = t
+def _keep_host_constant(key, t: Tensor) -> Tensor:
+    if type(t) is Tensor and t.data_ptr() != 0 and len(_HOST_CONSTANTS) < 256:
+        _HOST_CONSTANTS[key] = t
     return t
 
 
