@@ -26,7 +26,7 @@
  *   - Per-device state (kernel attributes, the tm_edt_noalloc scratch
  *     address) is cached for the life of the process: calling
  *     cudaDeviceReset() on a device while the library is loaded is not
- *     supported.
+ *     supported.  Calls from several threads may run at the same time.
  */
 #ifndef TORCHMORPH_GB300_H
 #define TORCHMORPH_GB300_H
@@ -219,8 +219,8 @@ int tm_binary_dilation(const uint8_t *in, uint8_t *out, int64_t batch, int ndim,
  * a structure of more than 128 voxels), where the caller composes the
  * operators.  tm_binary_erosion / tm_binary_dilation of 3-D items run on the
  * same tiles within these limits.
- * 1-D / 2-D tm_binary_erosion / tm_binary_dilation with elements other than
- * full boxes run on the same bit tiles. */
+ * 1-D / 2-D tm_binary_erosion / tm_binary_dilation run on the same bit tiles,
+ * but for full boxes of more than 65 voxels. */
 int tm_binary_opening(const uint8_t *in, uint8_t *out, int64_t batch, int ndim, const int64_t *shape,
                       const uint8_t *structure, const int64_t *sshape, const int64_t *origin,
                       int border_value, tm_stream_t stream);

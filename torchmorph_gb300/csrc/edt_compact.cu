@@ -1698,9 +1698,11 @@ int edt_compact_run(const void *input, int in_dtype, const Geometry &g, const Ed
     int16_t *c1 = reinterpret_cast<int16_t *>(ws);
     int32_t *c2 = g.ndim == 3 ? reinterpret_cast<int32_t *>(ws + align256(n * 2)) : nullptr;
     // Rows up to 256 take the search whatever the plane's size, longer ones in planes of less
-    // than 50 K voxels: 2 x 160 x 160 x 256, background 50 / 10 / 1 / 0.1 %, passes alone 145 /
-    // 150 / 185 / 338 us, search first 78 / 99 / 246 / 435 us; 64 x 250 x 512 94 / 98 us against
-    // 87 / 130.
+    // than 50 K voxels.  It pays on dense backgrounds and costs on sparse ones, which no host
+    // knows apart: 2 x 160 x 160 x 256 with features, background 50 / 10 / 1 / 0.1 %, passes
+    // alone 119 / 125 / 163 / 316 us, search first 64 / 87 / 226 / 416 (one thread per line,
+    // before: 125 / 147 / 1204 / 986); 4 x 128^3 78 / 82 / 109 / 219 and 34 / 38 / 240 / 270.
+    // 64 x 250 x 512, 50 / 10 %: passes 77 / 80 us, search first 87 / 130.
     const bool shell_shape = g.ndim == 3 && !spacing.scaled && p.L0 <= 254 && p.L1 <= 254 && (p.L2 % 4) == 0 &&
                              ((uintptr_t)dist & 15) == 0 && ((uintptr_t)indices & 15) == 0 &&
                              ((uintptr_t)sqdist & 15) == 0 && (g.numel % 4) == 0 &&

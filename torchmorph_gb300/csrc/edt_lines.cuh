@@ -26,9 +26,9 @@
 //
 // Bound: issue (about 190 instructions per voxel and pass on masks) and the latency of
 // the list phases, not memory: 8 x 1000 x 1333 masks, distances alone, move 64 MB in
-// 107 us.  Before (one thread, or one warp's lane 0, per line's envelope): 1217 us; 2 x 88 x
-// 180 x 214 at spacing (2.5, 1, 1) 1152 -> 149 us; 4 x 128^3 with features, masks 790 ->
-// 272 us, Bernoulli(0.99) 623 -> 250 us.  Windows decided per warp instead of by lists
+// 98 us.  Before (one thread, or one warp's lane 0, per line's envelope): 1217 us; 2 x 88 x
+// 180 x 214 at spacing (2.5, 1, 1) 1152 -> 126 us; 4 x 128^3 with features, masks 748 ->
+// 275 us, Bernoulli(0.99) 629 -> 239 us.  Windows decided per warp instead of by lists
 // (a warp runs the widest ring any of its lanes needs) took 138 us on the 2-D masks;
 // open positions walked inside their group's thread 121 us.
 //
