@@ -40,7 +40,7 @@ constexpr int kQB = 8;               // pass 1 outputs per register window
 constexpr int kSqrtTab = 64;         // correctly rounded sqrt of 0..63 in shared memory
 constexpr int kMaxL1 = 1024;          // axis 1 of 3-D items: 32 staged columns (200 KB)
 constexpr int kMaxL2 = 4096;          // last axis: 8 staged rows (198 KB)
-constexpr int kShortLine = 128;       // rows up to this length are staged 32 at a time
+constexpr int kShortLine = 128;       // rows up to this length are staged 32 or 16 at a time
 constexpr int kMediumLine = 512;      // longer rows take 512 threads per tile
 
 struct CompactParams {
@@ -1769,7 +1769,7 @@ int edt_compact_run(const void *input, int in_dtype, const Geometry &g, const Ed
     int st = in_dtype == TM_F32 ? launch_bits0(static_cast<const float *>(input), c1, p, todo, stream)
                                 : launch_bits0(static_cast<const uint8_t *>(input), c1, p, todo, stream);
     if (st != TM_OK) return st;
-    // lines per tile: 8 long rows, 32 short ones or columns; 512 threads where the staged
+    // lines per tile: 8 long rows, 16 or 32 short ones, 32 columns; 512 threads where the staged
     // lines (68 KB at 1333 voxels) leave room for few CTAs
     auto rows = [&](auto mode, auto out, const void *src, int L) -> int {
         constexpr int M = decltype(mode)::value, O = decltype(out)::value;

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(T, 1024 / T) edt_line_kernel(const void *__res
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int kSlots = T / NL;
     // list entries: line and group of 8 positions, line and position (32 lines reach 1024
-    // positions, 8 reach 4096)
+    // positions, 16 reach 2048, 8 reach 4096)
     constexpr int kPosBits = NL == 32 ? 10 : (NL == 16 ? 11 : 12), kPosMask = (1 << kPosBits) - 1;
     constexpr int kTaskBits = kPosBits - 3, kTaskMask = (1 << kTaskBits) - 1;
     const int L = MODE == 2 ? p.L2 : p.L1;
